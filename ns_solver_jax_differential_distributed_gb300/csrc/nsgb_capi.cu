@@ -86,6 +86,7 @@ struct nsgb_plan {
   int device = 0;
   float2* tw = nullptr;
   float* k2 = nullptr;
+  float scale = 0.f;  // of the Poisson multiplier (fft::host_wavenumbers)
   int tile_w = 64, tile_h = 16, rows_per_cta = 8, cols_per_cta = 2;
   int adj_w = 64, adj_h = 16;  // tiled-kernel shape of the adjoint stencil
   int radix_rows = 16, radix_cols = 16;  // Stockham radix of the FFT passes
@@ -200,7 +201,7 @@ FftLaunch fft_launch(const nsgb_plan* plan, const float* rhs, void* spec, float*
   L.p = p;
   L.tw = plan->tw;
   L.k2 = plan->k2;
-  L.scale = (float)(1.0 / (2.0 * (double)plan->N * (double)plan->N));
+  L.scale = plan->scale;
   L.rows_per_cta = plan->rows_per_cta;
   L.cols_per_cta = plan->cols_per_cta;
   L.radix_rows = plan->radix_rows;
@@ -897,19 +898,8 @@ int nsgb_plan_create(int N, double L, nsgb_plan** out) {
   const int ntw = nsgb::fft::tw_total(N);
   std::vector<float2> tw(ntw);
   nsgb::fft::host_twiddles(N, tw.data());
-  // k = 2 pi fftfreq(N, dx) in float32 as NS_solver.py:518-519 evaluates it:
-  // (m / float32(dx*N)) * 2 * float32(pi), then squared in float32.
   std::vector<float> k2(N);
-  const double dx = L / N;
-  const float dn = (float)(dx * N);
-  for (int m = 0; m < N; ++m) {
-    const int mm = m < N / 2 ? m : m - N;
-    volatile float k = (float)mm / dn;
-    k = k * 2.0f;
-    k = k * (float)M_PI;
-    volatile float kk = k * k;
-    k2[m] = kk;
-  }
+  nsgb::fft::host_wavenumbers(N, L, k2.data(), &p->scale);
   cudaError_t e = cudaMalloc(&p->tw, ntw * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&p->k2, N * sizeof(float));
   if (e == cudaSuccess) e = cudaMemcpy(p->tw, tw.data(), ntw * sizeof(float2), cudaMemcpyHostToDevice);
@@ -2142,7 +2132,7 @@ int nsgb_ensemble_persistent(const nsgb_member* members_in, int count, void* wor
       a.jpart_rows = steps;
     }
     const int N = x.plan->N;
-    pm[k] = {x.plan->tw, x.plan->k2, (float)(1.0 / (2.0 * (double)N * (double)N)), N};
+    pm[k] = {x.plan->tw, x.plan->k2, x.plan->scale, N};
     int it[4];
     pers_items(N, it);
     for (int s = 0; s < 4; ++s) first[(size_t)s * (count + 1) + k + 1] = first[(size_t)s * (count + 1) + k] + it[s];

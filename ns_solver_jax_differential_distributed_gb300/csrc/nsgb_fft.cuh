@@ -19,6 +19,7 @@
 // followed by the radix-8 tables (host_twiddles).
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 
 #include "nsgb_common.cuh"
@@ -134,6 +135,30 @@ inline void host_twiddles(int N, float2* out) {
         }
     }
   }
+}
+
+// Squared wavenumbers k2[m] (N entries) and the factor `scale` such that the
+// Poisson multiplier is -scale / (k2[a] + k2[b]).  k = 2 pi fftfreq(N, dx) in
+// float32 as NS_solver.py:518-519 evaluates it: (m / float32(dx*N)) * 2 *
+// float32(pi), then squared in float32; then scaled by the power of two that
+// brings k2[1] to [1, 2) (exact, as are the 1/2 of the two-for-one split and
+// the 1/N^2 of the inverse transform in `scale`), so that every sum of two
+// entries lies well inside the range of the kernels' reciprocal.
+inline void host_wavenumbers(int N, double L, float* k2, float* scale) {
+  const double dx = L / N;
+  const float dn = (float)(dx * N);
+  for (int m = 0; m < N; ++m) {
+    const int mm = m < N / 2 ? m : m - N;
+    volatile float k = (float)mm / dn;
+    k = k * 2.0f;
+    k = k * (float)M_PI;
+    volatile float kk = k * k;
+    k2[m] = kk;
+  }
+  int e = 0;
+  if (k2[1] > 0.0f && std::isfinite(k2[1])) e = std::min(100, std::max(-100, -std::ilogb(k2[1])));
+  for (int m = 0; m < N; ++m) k2[m] = (float)std::ldexp((double)k2[m], e);
+  *scale = (float)std::ldexp(1.0 / (2.0 * (double)N * (double)N), e);
 }
 
 // a[s] = buffer[pad(j + s*T)], s = 0..E-1 (and the store of the same

@@ -69,12 +69,25 @@ __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, flo
 }
 
 // ----------------------------------------------------------------- columns --
-// Spectral multiplier  -1/(kx^2 + ky^2) * scale, 0 where the sum is 0.
+// Spectral multiplier  -1/(k2x + k2y) * scale, 0 where the sum is 0.  The
+// hardware reciprocal (within one ulp) and one Newton-Raphson step,
+// r' = r + r (1 - d r) with a fused residual, give the correctly rounded 1/d
+// (the same float as __frcp_rn for every mantissa) without that function's
+// range check, which kept the 16 multipliers of a thread from overlapping;
+// host_wavenumbers keeps d in [1, 2^28].  FAST = false (N = 8192, whose 64
+// registers per thread the overlap would overflow) calls __frcp_rn.
+template <bool FAST>
 __device__ __forceinline__ float poisson_mult(float k2x, float k2y, float scale) {
-  const float den = k2x + k2y;
-  // __frcp_rn is the correctly rounded 1/den, the same float as 1.0f / den
-  const float inv = (den == 0.0f) ? 0.0f : __frcp_rn(den);
-  return -inv * scale;
+  const float d = k2x + k2y;
+  if constexpr (FAST) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = __fmaf_rn(r, __fmaf_rn(-d, r, 1.0f), r);
+    return d > 0.0f && d < INFINITY ? -r * scale : 0.0f;
+  } else {
+    const float inv = d == 0.0f ? 0.0f : __frcp_rn(d);
+    return -inv * scale;
+  }
 }
 
 // Transform thread j of spectrum row y of a CTA carrying KB rows, rows
@@ -101,8 +114,14 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
   const float k2y = gldg(k2 + ky);
 #pragma unroll
   for (int s = 0; s < E; ++s) {
-    const float g = poisson_mult(gldg(k2 + j + s * T), k2y, scale);
-    a[s] = make_float2(a[s].x * g, a[s].y * g);
+    const float g = poisson_mult<(N < 8192)>(gldg(k2 + j + s * T), k2y, scale);
+    // From N = 2048 on the product may fuse into the inverse transform's first
+    // butterflies (39.6 against 43.0 us at N = 4096); below that the pass is not
+    // bound by arithmetic and rounds it on its own, as the reference does.
+    if constexpr (N >= 2048)
+      a[s] = make_float2(a[s].x * g, a[s].y * g);
+    else
+      a[s] = make_float2(__fmul_rn(a[s].x, g), __fmul_rn(a[s].y, g));
   }
   fft::block_fft<N, true, E>(a, sb, j, tw);
   __syncthreads();  // rows clamped to N/2 were loaded by other threads

@@ -23,15 +23,26 @@
 namespace nsgb {
 
 // ---------------------------------------------------------------- kernels --
-// Radix 16 keeps about 64 registers per thread; radix 8 about 40, so its
-// column kernel is bounded for three 512-thread CTAs per SM.
+// The column pass is bound by the FP32 pipe's operand bandwidth (a fused
+// multiply-add of three different registers issues at 0.64 of the rate of one
+// with two) and by shared memory; two CTAs of 256 threads per SM already
+// saturate both, so registers matter more than warps: the radix-16 kernel is
+// bounded to 80 registers (768 threads per SM), where the multipliers of a
+// thread overlap and little spills.  Times of the pass in the step: N = 4096
+// 46.4 -> 39.7 us, 1024 11.4 -> 8.2 us, 128 9.4 -> 6.3 us.  N = 8192 has CTAs of
+// 512 threads and needs two of them per SM (213 us, against 240 us for one with
+// 128 registers); so does radix 8, whose registers allow it.
+template <int N, int E>
+constexpr bool cols_two() {
+  return E == 8 || N >= 8192;
+}
 template <int N, int E>
 __global__ void __launch_bounds__(1024) k_rows_fwd(const float* __restrict__ rhs, float2* __restrict__ spec,
                                                    const float2* __restrict__ tw) {
   rows_fwd_body<N, E>(rhs, spec, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
 }
 template <int N, int E>
-__global__ void __launch_bounds__(512, E == 8 ? 3 : 2) k_cols(float2* __restrict__ spec,
+__global__ void __launch_bounds__(cols_two<N, E>() ? 512 : 768, cols_two<N, E>() ? 2 : 1) k_cols(float2* __restrict__ spec,
                                                               const float2* __restrict__ tw,
                                                               const float* __restrict__ k2, float scale) {
   cols_body<N, E>(spec, tw, k2, scale, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
@@ -49,7 +60,7 @@ __global__ void __launch_bounds__(1024) k_rows_fwd_b(const SolveDev* __restrict_
   rows_fwd_body<N, E>(f.rhs, f.spec, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
 }
 template <int N, int E>
-__global__ void __launch_bounds__(512, E == 8 ? 3 : 2) k_cols_b(const SolveDev* __restrict__ sv,
+__global__ void __launch_bounds__(cols_two<N, E>() ? 512 : 768, cols_two<N, E>() ? 2 : 1) k_cols_b(const SolveDev* __restrict__ sv,
                                                                 const float2* __restrict__ tw,
                                                                 const float* __restrict__ k2, float scale) {
   cols_body<N, E>(sv[blockIdx.y].fft.spec, tw, k2, scale, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);

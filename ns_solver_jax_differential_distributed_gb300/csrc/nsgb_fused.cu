@@ -69,8 +69,8 @@ struct Shape {
   static constexpr int STG_OFF = UY_OFF + kURing * RS;
   static constexpr int INV_OFF = STG_OFF + NSLOT * XB;
   static constexpr int EDGE_OFF = INV_OFF + XB;          // [2 slots][3 fields][2 sides][NWS]
-  static constexpr int RED_OFF = EDGE_OFF + 12 * NWS;    // 32 partial sums
-  static constexpr int F_OFF = RED_OFF + 32;             // f_x of rows r0-1 .. r1
+  static constexpr int RED_OFF = EDGE_OFF + 12 * NWS;    // 32 partial sums (double-float)
+  static constexpr int F_OFF = RED_OFF + 64;             // f_x of rows r0-1 .. r1
   static_assert(C <= 2, "clusters of one or two CTAs");
   static_assert(THREADS <= 1024, "block size");
   static_assert(XB % 4 == 0 && RS % 4 == 0 && (12 * NWS) % 4 == 0, "16-byte aligned sections");
@@ -245,7 +245,7 @@ __device__ __forceinline__ void fused_rows_body(const FusedArgs& fa) {
   float* sUX = sm + S::UX_OFF;
   float* sUY = sm + S::UY_OFF;
   float* sE = sm + S::EDGE_OFF;
-  float* sRed = sm + S::RED_OFF;
+  DFloat* sRed = reinterpret_cast<DFloat*>(sm + S::RED_OFF);
   float* sF = sm + S::F_OFF;
 
   const int step = (a.step_ctr ? gld(a.step_ctr) : 0) + a.step_fixed;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void fused_rows_body(const FusedArgs& fa) {
   // and y row t-2; rhs of the even row of the pending pair
   float u1x[4] = {0, 0, 0, 0}, u1y[4] = {0, 0, 0, 0}, u2x[4] = {0, 0, 0, 0}, u2y[4] = {0, 0, 0, 0};
   float sx3[4] = {0, 0, 0, 0}, sx2[4] = {0, 0, 0, 0}, sy2[4] = {0, 0, 0, 0}, rhe[4] = {0, 0, 0, 0};
-  float jacc = 0.0f;
+  ObjectiveSum jacc;
 
   auto iterate = [&](int t, int h, int k) {
     const int rs = (t - 1) & 1, ws = t & 1;
@@ -342,9 +342,7 @@ __device__ __forceinline__ void fused_rows_body(const FusedArgs& fa) {
         const size_t o = (size_t)((t - 2) & M) * N + col;
         st4_stream(uso_x, o, sx2);
         st4_stream(uso_y, o, sy2);
-        const float fj = sF[t - r0 - 1];
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) jacc += u2x[kk] * fj;
+        jacc.add(u2x, sF[t - r0 - 1], t);
         if (h == 0) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) rhe[kk] = rh[kk];
@@ -445,12 +443,12 @@ __device__ __forceinline__ void fused_rows_body(const FusedArgs& fa) {
   }
   // objective partial of the CTA
   cp_wait<0>();
-  jacc = warp_sum(jacc);
-  if (lane == 0) sRed[warp] = jacc;
+  const DFloat jsum = warp_sum_df(jacc.total());
+  if (lane == 0) sRed[warp] = jsum;
   fft::group_sync<1, ST>();
   if (warp == 0) {
-    float v = lane < NWS ? sRed[lane] : 0.0f;
-    v = warp_sum(v);
+    const DFloat z = {0.f, 0.f};
+    const float v = warp_sum_df(lane < NWS ? sRed[lane] : z).hi;
     if (lane == 0 && (unsigned)step < (unsigned)a.jpart_rows) {
       const int nblk = gridDim.x * gridDim.y;
       gst(a.jpart + (size_t)step * nblk + blockIdx.y * gridDim.x + blockIdx.x, v);

@@ -15,8 +15,8 @@ struct FftLaunch {
   bool do_cols = true;         // column transform + Poisson multiplier
   float* p = nullptr;          // rows inverse output (nullptr: skip the pass)
   const float2* tw = nullptr;  // per-pass twiddle tables (nsgb_fft.cuh)
-  const float* k2 = nullptr;   // squared wavenumbers, N entries
-  float scale = 0.f;           // 1 / (2 N^2)
+  const float* k2 = nullptr;   // squared wavenumbers, N entries (fft::host_wavenumbers)
+  float scale = 0.f;           // of the Poisson multiplier
   int rows_per_cta = 8;        // even, power of two
   int cols_per_cta = 2;        // power of two
   int radix_rows = 16;         // Stockham radix of the row passes (16 or 8)
@@ -113,7 +113,7 @@ cudaError_t poisson_fft_batch(int N, const FftLaunch& L, const SolveDev* solves,
 struct PersMember {
   const float2* tw;  // the member's plan twiddles (radix-16 tables first)
   const float* k2;
-  float scale;       // 1 / (2 N^2)
+  float scale;       // of the Poisson multiplier
   int N;
 };
 struct PersWork {

@@ -67,19 +67,13 @@ int fail(int code, const char* fmt, ...) {
 }
 
 // Twiddles of the Stockham passes and squared wavenumbers, laid out and
-// rounded exactly as a plan of the same (N, L) holds them.
-void fill_tables(int N, double L) {
+// rounded exactly as a plan of the same (N, L) holds them; the multiplier's
+// scale.
+float fill_tables(int N, double L) {
+  float scale;
   nsgb::fft::host_twiddles(N, g_host_tw);
-  const double dx = L / N;
-  const float dn = (float)(dx * N);
-  for (int m = 0; m < N; ++m) {
-    const int mm = m < N / 2 ? m : m - N;
-    volatile float k = (float)mm / dn;
-    k = k * 2.0f;
-    k = k * (float)M_PI;
-    volatile float kk = k * k;
-    g_host_k2[m] = kk;
-  }
+  nsgb::fft::host_wavenumbers(N, L, g_host_k2, &scale);
+  return scale;
 }
 
 }  // namespace
@@ -128,7 +122,7 @@ extern "C" int nsgb_poisson_noalloc(int N, double L, const float* rhs, float* p,
     if (r) return r;
     d.ready = true;
   }
-  fill_tables(N, L);
+  const float scale = fill_tables(N, L);
   // From pageable host memory these copies return once the data is staged,
   // so the static host tables may be refilled by the next call.
   e = cudaMemcpyToSymbolAsync(g_noalloc_tw, g_host_tw, sizeof(float2) * nsgb::fft::tw_total(N), 0,
@@ -144,7 +138,7 @@ extern "C" int nsgb_poisson_noalloc(int N, double L, const float* rhs, float* p,
   Lc.p = p;
   Lc.tw = d.tw;
   Lc.k2 = d.k2;
-  Lc.scale = (float)(1.0 / (2.0 * (double)N * (double)N));
+  Lc.scale = scale;
   Lc.rows_per_cta = N >= 1024 ? 4 : 8;
   Lc.cols_per_cta = 1;
   e = nsgb::poisson_fft(N, Lc, st);

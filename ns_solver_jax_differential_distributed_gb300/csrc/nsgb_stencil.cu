@@ -79,9 +79,9 @@ constexpr unsigned kWaitLimit = 1u << 22;  // mbarrier polls before a CTA gives 
 constexpr bool kBulkRows = false;
 
 // shared memory: rings, edges [2 slots][3 fields][2 sides][G], forcing rows,
-// 32 partial sums, then (8-byte aligned) kMbSlots + 1 mbarriers
+// 32 partial sums (double-float), then (8-byte aligned) kMbSlots + 1 mbarriers
 inline size_t floats_before_mbar(int N, int W, int RH) {
-  const size_t f = (size_t)(kPRing + 2 * kURing) * ring_stride(W) + (size_t)12 * groups(N, W) + RH + 2 + 32;
+  const size_t f = (size_t)(kPRing + 2 * kURing) * ring_stride(W) + (size_t)12 * groups(N, W) + RH + 2 + 64;
   return (f + 1) & ~(size_t)1;
 }
 inline size_t smem_bytes(int N, int W, int RH) {
@@ -119,12 +119,12 @@ __device__ __forceinline__ void stencil_rows_body(const StencilArgs& a, int step
   float* sUY = sUX + kURing * RS;              // [kURing][RS]
   float* sE = sUY + kURing * RS;               // [slot][field][side][G]
   float* sF = sE + 12 * G;                     // f_x of rows r0-1 .. r1
-  float* sRed = sF + RH + 2;                   // per-warp partial sums
+  DFloat* sRed = reinterpret_cast<DFloat*>(sF + RH + 2);  // per-warp partial sums
   auto edge = [&](int slot, int f, int side) { return sE + ((slot * 3 + f) * 2 + side) * G; };
   // mbarriers (BULK): [0, kMbSlots) the groups of iterations t (p row t+1,
   // u* row t) by (t - r0 + 2) mod kMbSlots, [kMbSlots] the prologue's p rows
   // r0-3, r0-2
-  uint64_t* sMb = reinterpret_cast<uint64_t*>(sm + (((kPRing + 2 * kURing) * (size_t)RS + (size_t)12 * G + RH + 2 + 32 + 1) & ~(size_t)1));
+  uint64_t* sMb = reinterpret_cast<uint64_t*>(sm + (((kPRing + 2 * kURing) * (size_t)RS + (size_t)12 * G + RH + 2 + 64 + 1) & ~(size_t)1));
 
   int step = (a.step_ctr ? gld(a.step_ctr) : 0) + a.step_fixed + step_off;
   const float t_now = a.t_from_step ? fmul((float)step, c.dt) : a.t_fixed;
@@ -209,7 +209,7 @@ __device__ __forceinline__ void stencil_rows_body(const StencilArgs& a, int step
   // and y row t-2
   float u1x[4] = {0, 0, 0, 0}, u1y[4] = {0, 0, 0, 0}, u2x[4] = {0, 0, 0, 0}, u2y[4] = {0, 0, 0, 0};
   float sx3[4] = {0, 0, 0, 0}, sx2[4] = {0, 0, 0, 0}, sy2[4] = {0, 0, 0, 0};
-  float jacc = 0.0f;
+  ObjectiveSum jacc;
   float* __restrict__ uso_x = a.us_out;
   float* __restrict__ uso_y = a.us_out + NN;
   float* __restrict__ rhs_g = a.rhs;
@@ -276,9 +276,7 @@ __device__ __forceinline__ void stencil_rows_body(const StencilArgs& a, int step
           st4(a.u_out, o, u2x);
           st4(a.u_out + NN, o, u2y);
         }
-        const float fj = sF[t - r0 - 1];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) jacc += u2x[k] * fj;
+        jacc.add(u2x, sF[t - r0 - 1], t);
       }
     }
 
@@ -324,13 +322,13 @@ __device__ __forceinline__ void stencil_rows_body(const StencilArgs& a, int step
   }
 
   // objective partial of the CTA
-  jacc = warp_sum(jacc);
+  const DFloat jsum = warp_sum_df(jacc.total());
   const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  if (lane == 0) sRed[warp] = jacc;
+  if (lane == 0) sRed[warp] = jsum;
   __syncthreads();
   if (warp == 0) {
-    float v = lane < nwarps ? sRed[lane] : 0.0f;
-    v = warp_sum(v);
+    const DFloat z = {0.f, 0.f};
+    float v = warp_sum_df(lane < nwarps ? sRed[lane] : z).hi;
     if (aborted) v = __int_as_float(0x7fc00000);  // NaN: the step did not complete
     if (lane == 0 && (unsigned)step < (unsigned)a.jpart_rows) {
       const int nblk = gridDim.x * gridDim.y;
