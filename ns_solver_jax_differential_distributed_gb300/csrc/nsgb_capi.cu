@@ -102,10 +102,27 @@ struct nsgb_plan {
 
 namespace {
 
-// Launch shapes measured best on GB300 by the autotuner (see autotune.py);
-// the autotuner refines them per process.
-void default_tiles(int N, int out[4]) {
+// Launch shapes of a plan that is not tuned; the autotuner (autotune.py)
+// refines them per process.
+//
+// Stencil: tiles up to N = 512, where a grid has too few rows for bands that
+// fill the GPU (N = 512: 8.4 us tiled, 9.4 us in bands); row bands from N = 1024
+// on (in the step, central, tiles of 64 x 16 against bands: N = 1024 14.4 ->
+// 12.4 us, 2048 39 -> 26.6, 4096 133 -> 70.1).  Bands of 1024 columns, two CTAs
+// per SM in one wave, while they are at least 8 rows tall (each recomputes four
+// rows of its neighbours; at N = 1024 one CTA per SM, 7 rows, beats two of 4
+// rows: 12.4 against 13.7 us); at N = 8192 bands of 2048 columns, one CTA per SM
+// (265 against 285 us).
+void default_tiles(int N, int sms, int out[4]) {
   tile_kernel_default(N, out[0], out[1]);
+  if (N >= 1024) {
+    out[0] = N >= 8192 ? 2048 : 1024;
+    for (int per_sm = N >= 8192 ? 1 : 2; per_sm >= 1; --per_sm) {
+      const int bands = std::max(1, per_sm * sms / (N / out[0]));
+      out[1] = (N + bands - 1) / bands;
+      if (out[1] >= 8) break;
+    }
+  }
   int rows = N >= 1024 ? 4 : (N >= 256 ? 8 : 16);
   if (rows > N) rows = N;
   out[2] = rows;
@@ -875,16 +892,16 @@ int nsgb_plan_create(int N, double L, nsgb_plan** out) {
   p->logN = ilog2(N);
   p->L = L;
   cudaGetDevice(&p->device);
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
   int t[4];
-  default_tiles(N, t);
+  default_tiles(N, sms, t);
   p->tile_w = t[0];
   p->tile_h = t[1];
   tile_kernel_default(N, p->adj_w, p->adj_h);
   if (N >= 1024) {
     // the row-streaming adjoint: bands of 1024 columns, rows for about two
     // CTAs per SM (measured faster than the tiles from N = 1024 on)
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
     const int col_bands = N / NSGB_ADJ_ROWS_MAX_W;
     const int row_bands = (2 * sms + col_bands - 1) / col_bands;
     p->adj_w = NSGB_ADJ_ROWS_MAX_W;
