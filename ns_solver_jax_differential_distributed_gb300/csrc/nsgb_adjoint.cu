@@ -111,6 +111,21 @@ __device__ __forceinline__ void forcing_theta_grad(int i, const ForcingRow& fr, 
   dB = dsig * (-2.0f * cb * sinf(argB) * twopi * t);
 }
 
+// Adds a block's theta sensitivities of one adjoint step to its running sums
+// (double, one triple per block, steps in backward order); the first adjoint
+// step (no lambda yet) starts them.  Keeping the sums per block leaves one
+// small reduction per gradient (launch_gsum).
+__device__ __forceinline__ void add_theta_partials(const AdjointArgs& a, int blk, DFloat v0, DFloat v1, DFloat v2) {
+  double* gp = a.gpart + (size_t)blk * 3;
+  const bool more = a.lam != nullptr;
+  const double w0 = (double)v0.hi + (double)v0.lo, w1 = (double)v1.hi + (double)v1.lo;
+  // the nu partial carries the Laplacian's 1/dx^2 and the step's dt
+  const double w2 = ((double)v2.hi + (double)v2.lo) * ((double)a.c.dt * (double)a.c.rdx2);
+  gst(gp, more ? gld(gp) + w0 : w0);
+  gst(gp + 1, more ? gld(gp + 1) + w1 : w1);
+  gst(gp + 2, more ? gld(gp + 2) + w2 : w2);
+}
+
 template <int SCHEME, int TW, int TH>
 __device__ __forceinline__ void adjoint_body(const AdjointArgs& a) {
   using Lay = AdjointSmem<TW, TH>;
@@ -245,12 +260,7 @@ __device__ __forceinline__ void adjoint_body(const AdjointArgs& a) {
     const DFloat v1 = warp_sum_df(tx < 8 ? sRed[8 + tx] : z);
     const DFloat v2 = warp_sum_df(tx < 8 ? sRed[16 + tx] : z);
     if (tx == 0) {
-      const int nblk = gridDim.x * gridDim.y;
-      double* gp = a.gpart + ((size_t)a.gslot * nblk + blockIdx.y * gridDim.x + blockIdx.x) * 3;
-      gst(gp, (double)v0.hi + (double)v0.lo);
-      gst(gp + 1, (double)v1.hi + (double)v1.lo);
-      // the nu partial carries the Laplacian's 1/dx^2 and the step's dt
-      gst(gp + 2, ((double)v2.hi + (double)v2.lo) * ((double)dt * (double)c.rdx2));
+      add_theta_partials(a, blockIdx.y * gridDim.x + blockIdx.x, v0, v1, v2);
     }
   }
 }
@@ -531,11 +541,7 @@ __device__ __forceinline__ void adjoint_rows_body(const AdjointArgs& a) {
     const DFloat v1 = warp_sum_df(lane < nwarps ? sRed[adjrows::kMaxWarps + lane] : z);
     const DFloat v2 = warp_sum_df(lane < nwarps ? sRed[2 * adjrows::kMaxWarps + lane] : z);
     if (lane == 0) {
-      const int nblk = gridDim.x * gridDim.y;
-      double* gp = a.gpart + ((size_t)a.gslot * nblk + blockIdx.y * gridDim.x + blockIdx.x) * 3;
-      gst(gp, (double)v0.hi + (double)v0.lo);
-      gst(gp + 1, (double)v1.hi + (double)v1.lo);
-      gst(gp + 2, ((double)v2.hi + (double)v2.lo) * ((double)dt * (double)c.rdx2));
+      add_theta_partials(a, blockIdx.y * gridDim.x + blockIdx.x, v0, v1, v2);
     }
   }
 }
@@ -588,54 +594,25 @@ cudaError_t launch_adjoint_batch(const AdjointArgs& shape, const AdjointArgs* ta
   return launch_adjoint_any(shape, tab, count, st);
 }
 
-// Fixed-order reduction of nrows x nblk x 3 partials into gacc[3] (double):
-// one CTA per row sums the row's blocks by a fixed tree, then one thread adds
-// the row sums to gacc in row order.
-__global__ void k_greduce_rows(const double* __restrict__ gpart, int nblk, double* __restrict__ rowsum) {
+// dJ/dtheta from the blocks' sums, in a fixed order.
+__global__ void k_gsum(const double* __restrict__ gpart, int nblk, int theta_len, float* __restrict__ dJ) {
   __shared__ double red[3][256];
-  const double* base = gpart + (size_t)blockIdx.x * nblk * 3;
-  double v0 = 0, v1 = 0, v2 = 0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-    v0 += gld(base + 3 * b);
-    v1 += gld(base + 3 * b + 1);
-    v2 += gld(base + 3 * b + 2);
-  }
-  red[0][threadIdx.x] = v0;
-  red[1][threadIdx.x] = v1;
-  red[2][threadIdx.x] = v2;
+  const int t = threadIdx.x;
+  double v[3] = {0, 0, 0};
+  for (int b = t; b < nblk; b += 256)
+    for (int k = 0; k < 3; ++k) v[k] += gld(gpart + 3 * (size_t)b + k);
+  for (int k = 0; k < 3; ++k) red[k][t] = v[k];
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + s];
-      red[1][threadIdx.x] += red[1][threadIdx.x + s];
-      red[2][threadIdx.x] += red[2][threadIdx.x + s];
-    }
+  for (int h = 128; h > 0; h >>= 1) {
+    if (t < h)
+      for (int k = 0; k < 3; ++k) red[k][t] += red[k][t + h];
     __syncthreads();
   }
-  if (threadIdx.x < 3) gst(rowsum + 3 * blockIdx.x + threadIdx.x, red[threadIdx.x][0]);
+  if (t < theta_len) gst(dJ + t, (float)red[t][0]);
 }
 
-__global__ void k_greduce_acc(const double* __restrict__ rowsum, int nrows, double* __restrict__ gacc) {
-  if (threadIdx.x >= 3) return;
-  double g = gld(gacc + threadIdx.x);
-  for (int row = 0; row < nrows; ++row) g += gld(rowsum + 3 * row + threadIdx.x);
-  gst(gacc + threadIdx.x, g);
-}
-
-cudaError_t launch_greduce(const double* gpart, int nblk, int nrows, double* rowsum, double* gacc,
-                           cudaStream_t st) {
-  if (nrows <= 0) return cudaSuccess;
-  k_greduce_rows<<<nrows, 256, 0, st>>>(gpart, nblk, rowsum);
-  k_greduce_acc<<<1, 32, 0, st>>>(rowsum, nrows, gacc);
-  return cudaGetLastError();
-}
-
-__global__ void k_gfinal(const double* __restrict__ gacc, int theta_len, float* __restrict__ dJ) {
-  for (int k = 0; k < theta_len; ++k) gst(dJ + k, (float)gld(gacc + k));
-}
-
-cudaError_t launch_gfinal(const double* gacc, int theta_len, float* dJ, cudaStream_t st) {
-  k_gfinal<<<1, 1, 0, st>>>(gacc, theta_len, dJ);
+cudaError_t launch_gsum(const double* gpart, int nblk, int theta_len, float* dJ, cudaStream_t st) {
+  k_gsum<<<1, 256, 0, st>>>(gpart, nblk, theta_len, dJ);
   return cudaGetLastError();
 }
 

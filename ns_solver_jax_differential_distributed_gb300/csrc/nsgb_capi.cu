@@ -290,14 +290,9 @@ RolloutWs carve_rollout(const nsgb_plan* plan, int steps, void* ws) {
 struct GradWs {
   RolloutWs f;
   float *ckpt, *ustore, *lamA, *lamB, *padj;
-  double *gpart, *growsum, *gacc;
+  double* gpart;
   size_t bytes;
 };
-
-// Rows of per-block theta partials (one row per adjoint step) reduced into
-// the double accumulator by one launch: the summation order is the same for
-// every checkpoint interval.
-constexpr int kGradRows = 64;
 
 GradWs carve_grad(const nsgb_plan* plan, int steps, int every, void* ws) {
   const size_t NN = (size_t)plan->N * plan->N;
@@ -312,9 +307,7 @@ GradWs carve_grad(const nsgb_plan* plan, int steps, int every, void* ws) {
   g.lamA = cv.take<float>(2 * NN);
   g.lamB = cv.take<float>(2 * NN);
   g.padj = cv.take<float>(NN);
-  g.gpart = cv.take<double>((size_t)kGradRows * nblk * 3);
-  g.growsum = cv.take<double>((size_t)kGradRows * 3);
-  g.gacc = cv.take<double>(4);
+  g.gpart = cv.take<double>((size_t)nblk * 3);
   g.bytes = cv.off;
   return g;
 }
@@ -1338,7 +1331,6 @@ int grad_enqueue(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, 
 
   // Backward: segments in reverse; recompute each segment's states from its
   // checkpoint, then run the adjoint steps backwards through them.
-  NSGB_CUDA(cudaMemsetAsync(g.gacc, 0, 4 * sizeof(double), st));
   AdjointArgs b;
   b.c = a.c;
   b.scheme = a.scheme;
@@ -1352,7 +1344,6 @@ int grad_enqueue(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, 
   const float* lam = nullptr;  // lambda_S = 0
   bool have_padj = false;
   const int nseg = (steps + every - 1) / every;
-  int grow = 0;  // rows of gpart holding partials not yet reduced
   for (int seg = nseg - 1; seg >= 0; --seg) {
     const int s0 = seg * every, s1 = std::min(steps, s0 + every);
     const float* rc = g.ckpt + (size_t)seg * 2 * NN;
@@ -1373,12 +1364,7 @@ int grad_enqueue(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, 
       b.u = stored ? g.ckpt + (size_t)seg * 2 * NN : g.ustore + (size_t)(s - s0) * 2 * NN;
       b.lam_out = lam_out;
       b.step = s;
-      b.gslot = grow;
       NSGB_CUDA(launch_adjoint_stencil(b, st));
-      if (++grow == kGradRows) {
-        NSGB_CUDA(launch_greduce(g.gpart, adj_nblk, grow, g.growsum, g.gacc, st));
-        grow = 0;
-      }
       if (s > 0) {
         NSGB_CUDA(poisson_fft(plan->N, fft_launch(plan, w.rhs, w.spec, g.padj), st));
         have_padj = true;
@@ -1386,8 +1372,7 @@ int grad_enqueue(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, 
       lam = lam_out;
     }
   }
-  NSGB_CUDA(launch_greduce(g.gpart, adj_nblk, grow, g.growsum, g.gacc, st));
-  NSGB_CUDA(launch_gfinal(g.gacc, theta_len, dJdtheta, st));
+  NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
   return NSGB_OK;
 }
 }  // namespace
@@ -1560,9 +1545,9 @@ int check_grad_members(const nsgb_grad_member* m, int count) {
 
 // Work of one tick, enqueued after the tick's tables are on the device.
 struct GradAction {
-  enum Kind { GACC_ZERO, FWD, ADJ, GREDUCE, FFT, FWD_DONE, ADJ_DONE } kind;
+  enum Kind { FWD, ADJ, FFT, FWD_DONE, ADJ_DONE } kind;
   int group;           // plan group (its branch stream)
-  int member;          // GACC_ZERO, GREDUCE, FWD_DONE, ADJ_DONE
+  int member;          // FWD_DONE, ADJ_DONE
   const nsgb_plan* plan;
   int scheme;
   size_t off;          // FWD, ADJ, FFT: table offset in the upload
@@ -1642,7 +1627,6 @@ AdjointArgs grad_adj_args(const nsgb_grad_member& m, const GradMemberCtx& c, con
   x.u = (o.s1 - o.s0 == 1) ? c.g.ckpt + (size_t)o.seg * 2 * c.NN : c.g.ustore + (size_t)(s - o.s0) * 2 * c.NN;
   x.lam_out = (s == 0 && m.dJdu0) ? m.dJdu0 : ((b % 2 == 0) ? c.g.lamA : c.g.lamB);
   x.step = s;
-  x.gslot = b % kGradRows;
   return x;
 }
 
@@ -1705,7 +1689,7 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
       while (g1 < count && members[order[g1]].plan == plan) ++g1;
       std::vector<SolveDev> fwd[2], fft;
       std::vector<AdjointArgs> adj[2];
-      std::vector<GradAction> mid, post;
+      std::vector<GradAction> post;
       const size_t first_act = acts.size();
       for (int q = g0; q < g1; ++q) {
         const int i = order[q];
@@ -1714,12 +1698,6 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
         const GradMemberCtx& c = ctx[i];
         const GradOp o = grad_op(m.steps, m.every, m.done_ops + k);
         const int sch = m.phys.scheme == NSGB_SCHEME_CENTRAL ? 0 : 1;
-        if (m.done_ops + k == m.steps) {
-          GradAction z{};
-          z.kind = GradAction::GACC_ZERO;
-          z.member = i;
-          acts.push_back(z);
-        }
         if (o.kind != GOP_ADJ) {
           bool do_fft = false;
           const float* out_us = nullptr;
@@ -1740,13 +1718,6 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
           }
         } else {
           adj[sch].push_back(grad_adj_args(m, c, o));
-          const int b = m.steps - 1 - o.s;
-          if (b % kGradRows == kGradRows - 1) {
-            GradAction z{};
-            z.kind = GradAction::GREDUCE;
-            z.member = i;
-            mid.push_back(z);
-          }
           if (o.s > 0) {
             SolveDev f{};
             f.fft = {c.g.f.rhs, (float2*)c.g.f.spec, c.g.padj};
@@ -1779,7 +1750,6 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
         z.count = (int)adj[sch].size();
         acts.push_back(z);
       }
-      acts.insert(acts.end(), mid.begin(), mid.end());
       if (!fft.empty()) {
         GradAction z{};
         z.kind = GradAction::FFT;
@@ -1802,9 +1772,6 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
   for (const GradAction& z : acts) {
     cudaStream_t st = br.stream(z.group);
     switch (z.kind) {
-      case GradAction::GACC_ZERO:
-        NSGB_CUDA(cudaMemsetAsync(ctx[z.member].g.gacc, 0, 4 * sizeof(double), st));
-        break;
       case GradAction::FWD:
         NSGB_CUDA(launch_stencil_batch((const SolveDev*)(dev + z.off), z.count, 0, 0, z.scheme, z.plan->N,
                                        z.plan->tile_w, z.plan->tile_h, st));
@@ -1812,11 +1779,6 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
       case GradAction::ADJ:
         NSGB_CUDA(launch_adjoint_batch(z.shape, (const AdjointArgs*)(dev + z.off), z.count, st));
         break;
-      case GradAction::GREDUCE: {
-        const GradMemberCtx& c = ctx[z.member];
-        NSGB_CUDA(launch_greduce(c.g.gpart, c.adj_nblk, kGradRows, c.g.growsum, c.g.gacc, st));
-        break;
-      }
       case GradAction::FFT:
         NSGB_CUDA(poisson_fft_batch(z.plan->N, fft_launch(z.plan, nullptr, nullptr, nullptr),
                                     (const SolveDev*)(dev + z.off), z.count, st));
@@ -1832,8 +1794,7 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
       case GradAction::ADJ_DONE: {
         const nsgb_grad_member& m = members[z.member];
         const GradMemberCtx& c = ctx[z.member];
-        NSGB_CUDA(launch_greduce(c.g.gpart, c.adj_nblk, m.steps % kGradRows, c.g.growsum, c.g.gacc, st));
-        NSGB_CUDA(launch_gfinal(c.g.gacc, m.theta_len, m.dJdtheta, st));
+        NSGB_CUDA(launch_gsum(c.g.gpart, c.adj_nblk, m.theta_len, m.dJdtheta, st));
         break;
       }
     }

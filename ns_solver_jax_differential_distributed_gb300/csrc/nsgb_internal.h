@@ -158,11 +158,10 @@ struct AdjointArgs {
   const float* u = nullptr;      // (2,N,N) forward state u_s
   float* lam_out = nullptr;      // (2,N,N) lambda_s
   float* rhs = nullptr;          // (N,N) div(lambda_s)/dt
-  double* gpart = nullptr;       // per-block partial theta sensitivities, [step][nblk][3]
+  double* gpart = nullptr;       // per-block running theta sensitivities, [nblk][3]
   const float* theta = nullptr;
   int theta_len = 2;
   int step = 0;                  // forward step index s (forcing time t = s*dt)
-  int gslot = 0;                 // row of gpart to write
   int scheme = 0;
   int tw = 64, th = 16;
   StepConsts c;
@@ -178,10 +177,8 @@ cudaError_t launch_adjoint_batch(const AdjointArgs& shape, const AdjointArgs* ta
 // its five input rings bound the band) by th rows.
 constexpr int NSGB_ADJ_ROWS_MAX_W = 1024;
 bool adjoint_rows_supported(int N, int tw, int th);
-// rowsum: nrows x 3 doubles of scratch
-cudaError_t launch_greduce(const double* gpart, int nblk, int nrows, double* rowsum, double* gacc,
-                           cudaStream_t st);
-cudaError_t launch_gfinal(const double* gacc, int theta_len, float* dJ, cudaStream_t st);
+// dJ/dtheta from the nblk blocks' sums after the last adjoint step
+cudaError_t launch_gsum(const double* gpart, int nblk, int theta_len, float* dJ, cudaStream_t st);
 
 // ------------------------------------------------------------- optimiser --
 // Constants of one optimiser update, float32 as the library rounds them;

@@ -528,62 +528,83 @@ cudaError_t launch_project_batch(const SolveDev* solves, int count, int variant,
 }
 
 // ----------------------------------------------------------- J reduction --
-// One CTA per step: fixed-order sum of that step's block partials.
-__global__ void k_jreduce(const float* __restrict__ jpart, int nblk, double* __restrict__ jsteps) {
+// J = sum over steps of jscale * (sum of the step's block partials), in double
+// and in a fixed order: per step one warp up to kWarpBlocks blocks, else one CTA
+// (k_jreduce), then one CTA over the steps (k_jfinal; one thread adding 328
+// steps in turn took 8 us at the end of an N = 128 rollout).
+constexpr int kWarpBlocks = 1024;
+
+__device__ __forceinline__ void jreduce_body(const float* __restrict__ jpart, int nblk, int steps,
+                                             double* __restrict__ jsteps) {
   __shared__ double red[256];
+  const int t = threadIdx.x;
+  if (nblk <= kWarpBlocks) {
+    const int s = blockIdx.x * 8 + t / 32;
+    if (s >= steps) return;
+    const float* row = jpart + (size_t)s * nblk;
+    double v = 0.0;
+    for (int b = t % 32; b < nblk; b += 32) v += (double)gld(row + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (t % 32 == 0) gst(jsteps + s, v);
+    return;
+  }
   const float* row = jpart + (size_t)blockIdx.x * nblk;
   double v = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += (double)gld(row + b);
-  red[threadIdx.x] = v;
+  for (int b = t; b < nblk; b += 256) v += (double)gld(row + b);
+  red[t] = v;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+  for (int h = 128; h > 0; h >>= 1) {
+    if (t < h) red[t] += red[t + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) gst(jsteps + blockIdx.x, red[0]);
+  if (t == 0) gst(jsteps + blockIdx.x, red[0]);
+}
+static unsigned jreduce_grid(int nblk, int steps) { return nblk <= kWarpBlocks ? (steps + 7) / 8 : steps; }
+
+__device__ __forceinline__ void jfinal_body(const double* __restrict__ jsteps, int steps, double jscale,
+                                            float* __restrict__ J) {
+  __shared__ double red[256];
+  const int t = threadIdx.x;
+  double v = 0.0;
+  for (int s = t; s < steps; s += 256) v += gld(jsteps + s) * jscale;
+  red[t] = v;
+  __syncthreads();
+  for (int h = 128; h > 0; h >>= 1) {
+    if (t < h) red[t] += red[t + h];
+    __syncthreads();
+  }
+  if (t == 0) gst(J, (float)red[0]);
 }
 
-__global__ void k_jfinal(const double* __restrict__ jsteps, int steps, double jscale,
-                         float* __restrict__ J) {
-  double acc = 0.0;
-  for (int s = 0; s < steps; ++s) acc += gld(jsteps + s) * jscale;
-  gst(J, (float)acc);
+__global__ void __launch_bounds__(256) k_jreduce(const float* __restrict__ jpart, int nblk, int steps,
+                                                 double* __restrict__ jsteps) {
+  jreduce_body(jpart, nblk, steps, jsteps);
+}
+__global__ void __launch_bounds__(256) k_jfinal(const double* __restrict__ jsteps, int steps, double jscale,
+                                                float* __restrict__ J) {
+  jfinal_body(jsteps, steps, jscale, J);
 }
 
 cudaError_t launch_jreduce(const float* jpart, int nblk, int steps, double* jsteps, float* J,
                            double jscale, cudaStream_t st) {
-  if (steps > 0) k_jreduce<<<steps, 256, 0, st>>>(jpart, nblk, jsteps);
-  k_jfinal<<<1, 1, 0, st>>>(jsteps, steps, jscale, J);
+  if (steps > 0) k_jreduce<<<jreduce_grid(nblk, steps), 256, 0, st>>>(jpart, nblk, steps, jsteps);
+  k_jfinal<<<1, 256, 0, st>>>(jsteps, steps, jscale, J);
   return cudaGetLastError();
 }
 
-__global__ void k_jreduce_batch(const SolveDev* __restrict__ solves, int nblk) {
-  __shared__ double red[256];
+__global__ void __launch_bounds__(256) k_jreduce_batch(const SolveDev* __restrict__ solves, int nblk, int steps) {
   const SolveDev& d = solves[blockIdx.y];
-  const float* row = d.st[1].jpart + (size_t)blockIdx.x * nblk;
-  double v = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += (double)gld(row + b);
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) gst(d.jsteps + blockIdx.x, red[0]);
+  jreduce_body(d.st[1].jpart, nblk, steps, d.jsteps);
 }
-
-__global__ void k_jfinal_batch(const SolveDev* __restrict__ solves, int count, int steps) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const SolveDev& d = solves[k];
-  double acc = 0.0;
-  for (int s = 0; s < steps; ++s) acc += gld(d.jsteps + s) * d.jscale;
-  gst(d.J, (float)acc);
+__global__ void __launch_bounds__(256) k_jfinal_batch(const SolveDev* __restrict__ solves, int steps) {
+  const SolveDev& d = solves[blockIdx.x];
+  jfinal_body(d.jsteps, steps, d.jscale, d.J);
 }
 
 cudaError_t launch_jreduce_batch(const SolveDev* solves, int count, int nblk, int steps, cudaStream_t st) {
-  if (steps > 0) k_jreduce_batch<<<dim3(steps, count), 256, 0, st>>>(solves, nblk);
-  k_jfinal_batch<<<(count + 127) / 128, 128, 0, st>>>(solves, count, steps);
+  if (steps > 0) k_jreduce_batch<<<dim3(jreduce_grid(nblk, steps), count), 256, 0, st>>>(solves, nblk, steps);
+  k_jfinal_batch<<<count, 256, 0, st>>>(solves, steps);
   return cudaGetLastError();
 }
 
