@@ -546,12 +546,18 @@ __device__ __forceinline__ void adjoint_rows_body(const AdjointArgs& a) {
   }
 }
 
-template <int SCHEME>
-__global__ void __launch_bounds__(NSGB_ADJ_ROWS_MAX_W / 4 + 32) k_adjoint_rows(const AdjointArgs a) {
+// Bands up to 512 columns (at most 160 threads) run three CTAs per SM, which
+// the upwind kernel's 131 unbounded registers would cut to two; a band of 1024
+// columns fills the SM's shared memory with its rings and keeps its registers.
+constexpr int kNarrow = 512;
+template <int SCHEME, bool NARROW>
+__global__ void __launch_bounds__(NARROW ? kNarrow / 4 + 32 : NSGB_ADJ_ROWS_MAX_W / 4 + 32, NARROW ? 3 : 1)
+    k_adjoint_rows(const AdjointArgs a) {
   adjoint_rows_body<SCHEME>(a);
 }
-template <int SCHEME>
-__global__ void __launch_bounds__(NSGB_ADJ_ROWS_MAX_W / 4 + 32) k_adjoint_rows_b(const AdjointArgs* __restrict__ tab) {
+template <int SCHEME, bool NARROW>
+__global__ void __launch_bounds__(NARROW ? kNarrow / 4 + 32 : NSGB_ADJ_ROWS_MAX_W / 4 + 32, NARROW ? 3 : 1)
+    k_adjoint_rows_b(const AdjointArgs* __restrict__ tab) {
   adjoint_rows_body<SCHEME>(tab[blockIdx.z]);
 }
 
@@ -560,21 +566,29 @@ bool adjoint_rows_supported(int N, int tw, int th) {
   return th >= 1 && th <= N && adjrows::smem_bytes(N, rows::band_width(N, tw), th) <= 227 * 1024;
 }
 
-template <int SCHEME>
-static cudaError_t launch_adjoint_rows(const AdjointArgs& a, const AdjointArgs* tab, int count, cudaStream_t st) {
+template <int SCHEME, bool NARROW>
+static cudaError_t launch_adjoint_rows_t(const AdjointArgs& a, const AdjointArgs* tab, int count, int W,
+                                         cudaStream_t st) {
   const int N = a.c.N;
-  const int W = rows::band_width(N, a.tw);
   const size_t smem = adjrows::smem_bytes(N, W, a.th);
   if (smem > 48 * 1024) {
-    const cudaError_t e = tab ? raise_smem_limit(k_adjoint_rows_b<SCHEME>) : raise_smem_limit(k_adjoint_rows<SCHEME>);
+    const cudaError_t e =
+        tab ? raise_smem_limit(k_adjoint_rows_b<SCHEME, NARROW>) : raise_smem_limit(k_adjoint_rows<SCHEME, NARROW>);
     if (e != cudaSuccess) return e;
   }
   const dim3 grid(N / W, (N + a.th - 1) / a.th, tab ? count : 1);
   if (tab)
-    k_adjoint_rows_b<SCHEME><<<grid, rows::threads(N, W), smem, st>>>(tab);
+    k_adjoint_rows_b<SCHEME, NARROW><<<grid, rows::threads(N, W), smem, st>>>(tab);
   else
-    k_adjoint_rows<SCHEME><<<grid, rows::threads(N, W), smem, st>>>(a);
+    k_adjoint_rows<SCHEME, NARROW><<<grid, rows::threads(N, W), smem, st>>>(a);
   return cudaGetLastError();
+}
+
+template <int SCHEME>
+static cudaError_t launch_adjoint_rows(const AdjointArgs& a, const AdjointArgs* tab, int count, cudaStream_t st) {
+  const int W = rows::band_width(a.c.N, a.tw);
+  return W <= kNarrow ? launch_adjoint_rows_t<SCHEME, true>(a, tab, count, W, st)
+                      : launch_adjoint_rows_t<SCHEME, false>(a, tab, count, W, st);
 }
 
 static cudaError_t launch_adjoint_any(const AdjointArgs& a, const AdjointArgs* tab, int count, cudaStream_t st) {

@@ -893,12 +893,15 @@ int nsgb_plan_create(int N, double L, nsgb_plan** out) {
   p->tile_h = t[1];
   tile_kernel_default(N, p->adj_w, p->adj_h);
   if (N >= 1024) {
-    // the row-streaming adjoint: bands of 1024 columns, rows for about two
-    // CTAs per SM (measured faster than the tiles from N = 1024 on)
-    const int col_bands = N / NSGB_ADJ_ROWS_MAX_W;
-    const int row_bands = (2 * sms + col_bands - 1) / col_bands;
-    p->adj_w = NSGB_ADJ_ROWS_MAX_W;
-    p->adj_h = std::max(8, (N + row_bands - 1) / row_bands);
+    // The row-streaming adjoint, bands in one wave: 512 columns, three CTAs per
+    // SM, or at N = 1024 (too few rows for three) and N = 8192 1024 columns, one
+    // CTA per SM.  Backward step (adjoint stencil and FFT passes), upwind, 512
+    // against 1024 columns: N = 1024 29.4 / 25.0 us, 2048 69.6 / 76.6, 4096
+    // 230.8 / 234.5, 8192 1147 / 1056.
+    const bool wide = N == 1024 || N >= 8192;
+    p->adj_w = wide ? 1024 : 512;
+    const int bands = std::max(1, (wide ? 1 : 3) * sms / (N / p->adj_w));
+    p->adj_h = (N + bands - 1) / bands;
   }
   p->rows_per_cta = t[2];
   p->cols_per_cta = t[3];
