@@ -125,6 +125,24 @@ def _time_adjoint(u0, th, L, nu, dt, scheme, reps: int, steps: int = 6) -> float
     return e0.elapsed_time(e1) / (reps * steps)
 
 
+RESIDENT_MAX_N = 128  # largest grid of the resident kernel
+
+
+def _time_rollout(u0, th, L, nu, dt, scheme, steps: int = 64, reps: int = 3) -> float:
+    """Mean device ms per step of whole rollouts."""
+    def run():
+        return _native.op_rollout(u0, th, steps, L, nu, dt, _native.SCHEME_IDS[scheme], 0.5, 0.1, 1.0, True)
+    run()
+    torch.cuda.synchronize(u0.device)
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    for _ in range(reps):
+        run()
+    e1.record()
+    torch.cuda.synchronize(u0.device)
+    return e0.elapsed_time(e1) / (reps * steps)
+
+
 def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, reps: int = 5,
          force: bool = False, verbose: bool = False) -> dict:
     """Tune and apply the launch shapes of the plan (N, L, device)."""
@@ -181,6 +199,18 @@ def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, r
     best["ms"]["adjoint_step"] = results["adjoint"][(best["adj_tw"], best["adj_th"])]
     best["default"] += list(base_adj)
     plan.set_adjoint_tiles(best["adj_tw"], best["adj_th"])
+    # Small grids: whole rollouts run as one resident launch at the plan's first
+    # shapes only, which no stage timing sees; keep those if they win as a whole.
+    if N <= RESIDENT_MAX_N:
+        first = {"tw": base[0], "th": base[1], "rows": base[2], "cols": base[3], "radix_rows": base_radix[0],
+                 "radix_cols": base_radix[1], "adj_tw": base_adj[0], "adj_th": base_adj[1]}
+        tuned_ms = _time_rollout(u0, th, L, nu, dt, scheme)
+        _apply(plan, first)
+        first_ms = _time_rollout(u0, th, L, nu, dt, scheme)
+        if first_ms < tuned_ms:
+            best.update(first)
+        best["ms"]["rollout_step"] = min(first_ms, tuned_ms)
+        _apply(plan, best)
     if verbose:
         print(f"autotune N={N} {scheme}: best {best}")
         for kind, res in results.items():

@@ -659,6 +659,37 @@ cudaError_t rollout_step(const nsgb_plan* plan, StencilArgs a, const float* us_i
   return poisson_fft(plan->N, fft_launch(plan, w.rhs, w.spec, w.p), st);
 }
 
+// Whether a plan's rollouts (grad: and gradients) run as one resident launch:
+// N has an instance, the launch shapes are those it reproduces (32 x 8 tiles,
+// its radix), and the device can place its clusters.
+bool resident_plan(const nsgb_plan* plan, bool grad) {
+  const int radix = resident_radix(plan->N);
+  if (!radix || plan->radix_rows != radix || plan->radix_cols != radix) return false;
+  if (plan->tile_w != 32 || plan->tile_h != 8) return false;
+  if (grad && (plan->adj_w != 32 || plan->adj_h != 8)) return false;
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, bool> known;  // (N, device)
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(plan->N, plan->device);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  return known[key] = resident_available(plan->N);
+}
+
+ResidentArgs resident_args(const nsgb_plan* plan, const StencilArgs& a, const RolloutWs& w, int steps) {
+  ResidentArgs r;
+  r.c = a.c;
+  r.scheme = a.scheme;
+  r.tw = plan->tw + (resident_radix(plan->N) == 8 ? nsgb::fft::tw8_offset(plan->N) : 0);
+  r.k2 = plan->k2;
+  r.scale = plan->scale;
+  r.theta = a.theta;
+  r.theta_len = a.theta_len;
+  r.steps = steps;
+  r.jpart = w.jpart;
+  return r;
+}
+
 // Band width of the fused row kernel: whole rows up to 2048 columns, else
 // 2048-column slices (one CTA of a cluster each).
 int fused_width(int N) { return N / fused_cluster(N); }
@@ -719,6 +750,7 @@ cudaError_t bounds_upload_adjoint(const bounds::Table& t);
 cudaError_t bounds_upload_fused(const bounds::Table& t);
 cudaError_t bounds_upload_optim(const bounds::Table& t);
 cudaError_t bounds_upload_persistent(const bounds::Table& t);
+cudaError_t bounds_upload_resident(const bounds::Table& t);
 }  // namespace nsgb
 namespace {
 std::mutex g_bounds_mu;
@@ -744,7 +776,7 @@ int bounds_upload_locked() {
     }
   t.report = g_bounds_report;
   for (auto up : {bounds_upload_stencil, bounds_upload_fft, bounds_upload_adjoint, bounds_upload_fused,
-                  bounds_upload_optim, bounds_upload_persistent})
+                  bounds_upload_optim, bounds_upload_persistent, bounds_upload_resident})
     if ((e = up(t)) != cudaSuccess) return cuda_fail(e, "bounds table upload");
   return NSGB_OK;
 }
@@ -905,6 +937,7 @@ int nsgb_plan_create(int N, double L, nsgb_plan** out) {
   }
   p->rows_per_cta = t[2];
   p->cols_per_cta = t[3];
+  p->radix_rows = p->radix_cols = fft_default_radix(N);
 
   // Per-pass twiddle tables of the Stockham FFT, radix 16 then radix 8
   // (layout in nsgb_fft.cuh).
@@ -1200,6 +1233,16 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
     return finish_call(st);
   }
 
+  const double jscale = (double)phys->dt * (plan->L / plan->N) * (plan->L / plan->N);
+  if (resident_plan(plan, false)) {
+    ResidentArgs r = resident_args(plan, a, w, steps);
+    r.u0 = u0;
+    r.u_final = u_final;
+    NSGB_CUDA(launch_resident(plan->N, r, st));
+    NSGB_CUDA(launch_jreduce(w.jpart, nblk, steps, w.jsteps, J, jscale, st));
+    return finish_call(st);
+  }
+
   // step 0 reads u0 directly; later steps ping-pong usA <-> usB (and, fused,
   // the half spectrum spec <-> spec2).
   NSGB_CUDA(rollout_step(plan, a, u0, nullptr, w.usA, w, 0, nullptr, nullptr, !fused, st));
@@ -1295,8 +1338,7 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
     NSGB_CUDA(poisson_fft(plan->N, L, st));
   }
   NSGB_CUDA(launch_project(cur, w.p, u_final, a.c, st));
-  NSGB_CUDA(launch_jreduce(w.jpart, nblk, steps, w.jsteps, J, (double)phys->dt * (plan->L / plan->N) *
-                                                                  (plan->L / plan->N), st));
+  NSGB_CUDA(launch_jreduce(w.jpart, nblk, steps, w.jsteps, J, jscale, st));
   return finish_call(st);
 }
 
@@ -1315,6 +1357,26 @@ int grad_enqueue(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, 
   a.theta_len = theta_len;
   const int nblk = stencil_nblocks(plan->N, a.tw, a.th);
   const double dx = plan->L / plan->N;
+
+  if (resident_plan(plan, true)) {
+    ResidentArgs r = resident_args(plan, a, w, steps);
+    r.every = every;
+    r.phases = phases;
+    r.u0 = u0;
+    r.u_final = u_final;
+    r.ckpt = g.ckpt;
+    r.ustore = g.ustore;
+    r.lam = g.lamA;
+    r.padj = g.padj;
+    r.gpart = g.gpart;
+    r.dJdu0 = dJdu0;
+    NSGB_CUDA(launch_resident(plan->N, r, st));
+    if (phases & NSGB_GRAD_FORWARD)
+      NSGB_CUDA(launch_jreduce(w.jpart, nblk, steps, w.jsteps, J, (double)phys->dt * dx * dx, st));
+    if (phases & NSGB_GRAD_BACKWARD)
+      NSGB_CUDA(launch_gsum(g.gpart, stencil_nblocks(plan->N, plan->adj_w, plan->adj_h), theta_len, dJdtheta, st));
+    return NSGB_OK;
+  }
 
   if (phases & NSGB_GRAD_FORWARD) {
     // Forward rollout: checkpoint u_s every `every` steps, objective, u_final.
@@ -1404,6 +1466,11 @@ int nsgb_rollout_grad(const nsgb_plan* plan, const nsgb_phys* phys, const float*
   if (cap != cudaStreamCaptureStatusNone)
     return grad_enqueue(plan, phys, u0, theta, theta_len, steps, every, phases, J, u_final, dJdtheta, dJdu0,
                         workspace, st);  // (a capture is checked when it runs)
+  if (resident_plan(plan, true)) {  // three launches: nothing to gain from a graph
+    const int r = grad_enqueue(plan, phys, u0, theta, theta_len, steps, every, phases, J, u_final, dJdtheta, dJdu0,
+                               workspace, st);
+    return r ? r : finish_call(st);
+  }
   GradKey key;
   std::memset(&key, 0, sizeof key);
   key.ws = workspace;

@@ -187,13 +187,17 @@ __device__ __forceinline__ void store_strided(const float2 (&a)[E], float2* __re
   }
 }
 
-// Barrier of the threads that carry one transform: the whole CTA (BAR = 0)
-// or the NT threads of a warp group using hardware barrier BAR (kernels in
-// which other warps run other work at the same time).
+// Barrier of the threads that carry one transform: the whole CTA (BAR = 0),
+// the NT threads of a warp group using hardware barrier BAR (kernels in which
+// other warps run other work at the same time), or the warp (BAR = -1:
+// transforms of at most 32 threads, every lane of the warp calling).
 template <int BAR, int NT>
 __device__ __forceinline__ void group_sync() {
   if constexpr (BAR == 0) {
     __syncthreads();
+  } else if constexpr (BAR < 0) {
+    static_assert(NT <= 32, "a transform inside one warp");
+    __syncwarp();
   } else {
     asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NT) : "memory");
   }

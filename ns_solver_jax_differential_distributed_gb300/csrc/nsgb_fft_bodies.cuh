@@ -115,13 +115,9 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
 #pragma unroll
   for (int s = 0; s < E; ++s) {
     const float g = poisson_mult<(N < 8192)>(gldg(k2 + j + s * T), k2y, scale);
-    // From N = 2048 on the product may fuse into the inverse transform's first
-    // butterflies (39.6 against 43.0 us at N = 4096); below that the pass is not
-    // bound by arithmetic and rounds it on its own, as the reference does.
-    if constexpr (N >= 2048)
-      a[s] = make_float2(a[s].x * g, a[s].y * g);
-    else
-      a[s] = make_float2(__fmul_rn(a[s].x, g), __fmul_rn(a[s].y, g));
+    // (the products fuse into the inverse transform's first butterflies: 39.6
+    // against 43.0 us at N = 4096)
+    a[s] = make_float2(a[s].x * g, a[s].y * g);
   }
   fft::block_fft<N, true, E>(a, sb, j, tw);
   __syncthreads();  // rows clamped to N/2 were loaded by other threads

@@ -22,6 +22,10 @@ struct FftLaunch {
   int radix_rows = 16;         // Stockham radix of the row passes (16 or 8)
   int radix_cols = 16;         // ... and of the column pass
 };
+// Radix of a plan that is not tuned: 8 up to N = 128, where a step waits for the
+// transforms' latency (twice the threads share a transform), 16 above, where it
+// waits for shared memory (fewer exchanges).
+inline int fft_default_radix(int N) { return N >= 32 && N <= 128 ? 8 : 16; }
 cudaError_t poisson_fft(int N, const FftLaunch& L, cudaStream_t st);
 size_t fft_rows_smem_bytes(int N, int rows_per_cta);
 size_t fft_cols_smem_bytes(int N, int cols_per_cta);
@@ -179,6 +183,34 @@ constexpr int NSGB_ADJ_ROWS_MAX_W = 1024;
 bool adjoint_rows_supported(int N, int tw, int th);
 // dJ/dtheta from the nblk blocks' sums after the last adjoint step
 cudaError_t launch_gsum(const double* gpart, int nblk, int theta_len, float* dJ, cudaStream_t st);
+
+// --------------------------------------------------------------- resident --
+// A rollout or a gradient of a small grid in one cluster launch
+// (nsgb_resident.cu); the pointers are those of the batched path, which it
+// replaces value for value at 32 x 8 tiles.
+struct ResidentArgs {
+  StepConsts c;
+  int scheme = 0;
+  const float2* tw = nullptr;  // twiddles of the resident radix
+  const float* k2 = nullptr;
+  float scale = 0.f;
+  const float* theta = nullptr;
+  int theta_len = 2;
+  int steps = 0, every = 1;
+  int phases = 1;              // NSGB_GRAD_FORWARD | NSGB_GRAD_BACKWARD
+  const float* u0 = nullptr;   // forward
+  float* jpart = nullptr;      // objective partials, [step][tile]
+  float* u_final = nullptr;    // optional
+  float* ckpt = nullptr;       // checkpoints every `every` steps (nullptr: a plain rollout)
+  float* ustore = nullptr;     // a segment's states
+  float* lam = nullptr;        // lambda and its pressure while a segment is recomputed
+  float* padj = nullptr;
+  double* gpart = nullptr;     // theta sensitivities, [tile][3]
+  float* dJdu0 = nullptr;      // optional
+};
+int resident_radix(int N);        // radix of its transforms, 0: no instance for N
+bool resident_available(int N);   // the current device can launch its clusters
+cudaError_t launch_resident(int N, const ResidentArgs& a, cudaStream_t st);
 
 // ------------------------------------------------------------- optimiser --
 // Constants of one optimiser update, float32 as the library rounds them;
