@@ -459,9 +459,15 @@ static cudaError_t launch_stencil_s(const StencilArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
+// Tiles of eight rows, wider as the grid grows: up to N = 128 a wide tile leaves
+// SMs idle, at 512 and above (where only explicit-force steps and batches of
+// N = 512 use tiles) a narrow one loads half again its cells as halo.  Eleven
+// N = 512 solves in a batch, per step: 32 x 8 58.3 us, 64 x 8 48.5, 128 x 8 43.9
+// (one alone 14.3, 14.0, 14.2); its backward step 18.3, 15.9, 15.7.  N = 256, one
+// alone: 11.1 us for 32 and 64 wide, 12.1 for 128; backward 12.3, 12.0, 13.3.
 void tile_kernel_default(int N, int& tw, int& th) {
-  tw = N < 64 ? N : (N <= 512 ? 32 : 64);
-  th = N < 16 ? N : (N >= 1024 ? 16 : 8);
+  tw = N < 64 ? N : N <= 128 ? 32 : N <= 256 ? 64 : 128;
+  th = N < 16 ? N : 8;
 }
 
 cudaError_t launch_stencil(const StencilArgs& a, int mode, cudaStream_t st) {
