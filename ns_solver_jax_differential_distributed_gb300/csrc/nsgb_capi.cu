@@ -56,7 +56,6 @@ size_t spec_floats(int N) { return (size_t)(N / 2 + 1) * N * 2; }
 struct GraphEntry {
   const void* ws = nullptr;
   int steps = 0;
-  const float* theta = nullptr;
   int theta_len = 0;
   int chunk = 0;
   StepConsts c{};
@@ -65,18 +64,16 @@ struct GraphEntry {
   cudaGraphExec_t exec = nullptr;
 };
 
-// Everything a gradient call's enqueued work depends on (pointers are read at
-// replay, so a graph of the call replays it for the same arguments).
+// Everything the captured part of a gradient call depends on: its workspace
+// (whose theta slot the kernels read) and shapes, not the caller's buffers.
 struct GradKey {
   const void* ws;
-  const float *u0, *theta;
-  float *J, *u_final, *dJdtheta, *dJdu0;
-  int theta_len, steps, every, phases, scheme;
+  int part, theta_len, steps, every, scheme;
   int tiles[8];
   StepConsts c;
 };
 // compared with memcmp: no padding bytes
-static_assert(sizeof(GradKey) == 7 * sizeof(void*) + 13 * sizeof(int) + sizeof(StepConsts), "GradKey padding");
+static_assert(sizeof(GradKey) == sizeof(void*) + 13 * sizeof(int) + sizeof(StepConsts), "GradKey padding");
 
 }  // namespace
 
@@ -93,9 +90,9 @@ struct nsgb_plan {
   int fused_rows = 0;  // row band of the fused row kernel (0: the four-kernel step)
   cudaStream_t graph_stream = nullptr;  // private stream graphs are captured on
   std::vector<GraphEntry> graphs;
-  // gradient calls: the last call's arguments, and graphs of calls repeated
-  // with identical arguments
-  GradKey last_grad{};
+  // gradient calls: per part (forward, backward) the last call's key, and
+  // graphs of calls repeated with the same key
+  GradKey last_grad[2] = {};
   std::vector<std::pair<GradKey, cudaGraphExec_t>> grad_graphs;
   std::mutex mu;
 };
@@ -252,6 +249,7 @@ struct RolloutWs {
   float *usA, *usB, *p, *rhs, *spec, *spec2, *jpart;
   double* jsteps;
   int* ctr;
+  float* theta;  // the call's theta, at a fixed place for captured graphs
   int steps;  // rows of jpart
   size_t bytes;
 };
@@ -274,6 +272,7 @@ RolloutWs carve_rollout(const nsgb_plan* plan, int steps, void* ws) {
   // Buffers that captured graphs reference come first, at offsets that do
   // not depend on `steps`.
   w.ctr = cv.take<int>(1);
+  w.theta = (float*)w.ctr + 16;  // in the counter's 256 bytes
   w.usA = cv.take<float>(2 * NN);
   w.usB = cv.take<float>(2 * NN);
   w.p = cv.take<float>(NN);
@@ -1243,6 +1242,10 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
     return finish_call(st);
   }
 
+  // Graphs of a workspace serve any theta: the kernels read the call's copy.
+  NSGB_CUDA(cudaMemcpyAsync(w.theta, theta, theta_len * sizeof(float), cudaMemcpyDeviceToDevice, st));
+  a.theta = w.theta;
+
   // step 0 reads u0 directly; later steps ping-pong usA <-> usB (and, fused,
   // the half spectrum spec <-> spec2).
   NSGB_CUDA(rollout_step(plan, a, u0, nullptr, w.usA, w, 0, nullptr, nullptr, !fused, st));
@@ -1255,7 +1258,7 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
     std::lock_guard<std::mutex> lk(plan->mu);
     GraphEntry* ge = nullptr;
     for (auto& g : plan->graphs) {
-      if (g.ws == workspace && g.steps == steps && g.theta == theta && g.theta_len == theta_len && g.chunk == K &&
+      if (g.ws == workspace && g.steps == steps && g.theta_len == theta_len && g.chunk == K &&
           g.scheme == a.scheme && std::memcmp(&g.c, &a.c, sizeof(StepConsts)) == 0 &&
           g.tiles[0] == plan->tile_w && g.tiles[1] == plan->tile_h && g.tiles[2] == plan->rows_per_cta &&
           g.tiles[3] == plan->cols_per_cta && g.tiles[4] == plan->radix_rows &&
@@ -1290,7 +1293,6 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
       GraphEntry g;
       g.ws = workspace;
       g.steps = steps;
-      g.theta = theta;
       g.theta_len = theta_len;
       g.chunk = K;
       g.c = a.c;
@@ -1345,99 +1347,147 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
 }  // extern "C"
 
 namespace {
-// The work of one gradient call (validated arguments), enqueued on st.
-int grad_enqueue(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, const float* theta,
-                 int theta_len, int steps, int every, int phases, float* J, float* u_final, float* dJdtheta,
-                 float* dJdu0, void* workspace, cudaStream_t st) {
-  GradWs g = carve_grad(plan, steps, every, workspace);
-  const RolloutWs& w = g.f;
-  const size_t NN = (size_t)plan->N * plan->N;
-  StencilArgs a = stencil_args(plan, phys);
-  a.theta = theta;
-  a.theta_len = theta_len;
-  const int nblk = stencil_nblocks(plan->N, a.tw, a.th);
-  const double dx = plan->L / plan->N;
+// One gradient call (validated arguments).  Its launches that touch the
+// caller's buffers -- the first forward step, the final state, the objective,
+// the last adjoint step and the sensitivities -- are enqueued one by one; what
+// lies between them depends on the workspace alone and may replay as a graph.
+struct GradCall {
+  const nsgb_plan* plan;
+  const nsgb_phys* phys;
+  int theta_len, steps, every;
+  GradWs g;
+  StencilArgs a;
+  AdjointArgs b;
+  size_t NN;
 
-  if (resident_plan(plan, true)) {
-    ResidentArgs r = resident_args(plan, a, w, steps);
-    r.every = every;
-    r.phases = phases;
-    r.u0 = u0;
-    r.u_final = u_final;
-    r.ckpt = g.ckpt;
-    r.ustore = g.ustore;
-    r.lam = g.lamA;
-    r.padj = g.padj;
-    r.gpart = g.gpart;
-    r.dJdu0 = dJdu0;
-    NSGB_CUDA(launch_resident(plan->N, r, st));
-    if (phases & NSGB_GRAD_FORWARD)
-      NSGB_CUDA(launch_jreduce(w.jpart, nblk, steps, w.jsteps, J, (double)phys->dt * dx * dx, st));
-    if (phases & NSGB_GRAD_BACKWARD)
-      NSGB_CUDA(launch_gsum(g.gpart, stencil_nblocks(plan->N, plan->adj_w, plan->adj_h), theta_len, dJdtheta, st));
-    return NSGB_OK;
+  GradCall(const nsgb_plan* p, const nsgb_phys* ph, int theta_len_, int steps_, int every_, void* ws)
+      : plan(p), phys(ph), theta_len(theta_len_), steps(steps_), every(every_), g(carve_grad(p, steps_, every_, ws)),
+        a(stencil_args(p, ph)), NN((size_t)p->N * p->N) {
+    a.theta = g.f.theta;
+    a.theta_len = theta_len;
+    b.c = a.c;
+    b.scheme = a.scheme;
+    b.tw = plan->adj_w;
+    b.th = plan->adj_h;
+    b.theta = g.f.theta;
+    b.theta_len = theta_len;
+    b.gpart = g.gpart;
+    b.rhs = g.f.rhs;
   }
 
-  if (phases & NSGB_GRAD_FORWARD) {
-    // Forward rollout: checkpoint u_s every `every` steps, objective, u_final.
-    const float* cur = u0;
-    const float* curp = nullptr;
-    for (int s = 0; s < steps; ++s) {
-      float* out = (s % 2 == 0) ? w.usA : w.usB;
-      float* ck = (s % every == 0) ? g.ckpt + (size_t)(s / every) * 2 * NN : nullptr;
-      NSGB_CUDA(rollout_step(plan, a, cur, curp, out, w, s, nullptr, ck, true, st));
-      cur = out;
-      curp = w.p;
-    }
-    if (u_final) NSGB_CUDA(launch_project(cur, w.p, u_final, a.c, st));
-    NSGB_CUDA(launch_jreduce(w.jpart, nblk, steps, w.jsteps, J, (double)phys->dt * dx * dx, st));
+  // Forward step s from `in`: checkpoints u_s every `every` steps.
+  cudaError_t forward_step(int s, const float* in, cudaStream_t st) const {
+    float* out = (s % 2 == 0) ? g.f.usA : g.f.usB;
+    float* ck = (s % every == 0) ? g.ckpt + (size_t)(s / every) * 2 * NN : nullptr;
+    return rollout_step(plan, a, in, s == 0 ? nullptr : g.f.p, out, g.f, s, nullptr, ck, true, st);
   }
-  if (!(phases & NSGB_GRAD_BACKWARD)) return NSGB_OK;
+  const float* last_us() const { return (steps - 1) % 2 == 0 ? g.f.usA : g.f.usB; }
+
+  // Forward steps 1 .. steps - 1.
+  cudaError_t forward_rest(cudaStream_t st) const {
+    cudaError_t e = cudaSuccess;
+    for (int s = 1; s < steps && e == cudaSuccess; ++s)
+      e = forward_step(s, (s % 2 == 0) ? g.f.usB : g.f.usA, st);
+    return e;
+  }
+
+  // Adjoint step s (of segment seg, [s0, s1)): the n-th from the end reads and
+  // writes lambda in turns.
+  AdjointArgs adjoint_args(int s, int s0, int s1, float* dJdu0) const {
+    AdjointArgs x = b;
+    const int n = steps - 1 - s;
+    x.lam = n == 0 ? nullptr : (n % 2 == 1 ? g.lamA : g.lamB);
+    x.p = n == 0 ? nullptr : g.padj;
+    // a one-step segment's state is its checkpoint
+    x.u = s1 - s0 == 1 ? g.ckpt + (size_t)(s0 / every) * 2 * NN : g.ustore + (size_t)(s - s0) * 2 * NN;
+    x.lam_out = (s == 0 && dJdu0) ? dJdu0 : (n % 2 == 0 ? g.lamA : g.lamB);
+    x.step = s;
+    return x;
+  }
 
   // Backward: segments in reverse; recompute each segment's states from its
-  // checkpoint, then run the adjoint steps backwards through them.
-  AdjointArgs b;
-  b.c = a.c;
-  b.scheme = a.scheme;
-  b.tw = plan->adj_w;
-  b.th = plan->adj_h;
-  const int adj_nblk = stencil_nblocks(plan->N, b.tw, b.th);
-  b.theta = theta;
-  b.theta_len = theta_len;
-  b.gpart = g.gpart;
-  b.rhs = w.rhs;
-  const float* lam = nullptr;  // lambda_S = 0
-  bool have_padj = false;
-  const int nseg = (steps + every - 1) / every;
-  for (int seg = nseg - 1; seg >= 0; --seg) {
-    const int s0 = seg * every, s1 = std::min(steps, s0 + every);
-    const float* rc = g.ckpt + (size_t)seg * 2 * NN;
-    const float* rp = nullptr;
-    // a one-step segment's state is its checkpoint: nothing to recompute
-    const bool stored = (s1 - s0 == 1);
-    for (int s = s0; s < s1 && !stored; ++s) {
-      float* out = ((s - s0) % 2 == 0) ? w.usA : w.usB;
-      NSGB_CUDA(rollout_step(plan, a, rc, rp, out, w, s, nullptr, g.ustore + (size_t)(s - s0) * 2 * NN,
-                             s + 1 < s1, st));
-      rc = out;
-      rp = w.p;
-    }
-    for (int s = s1 - 1; s >= s0; --s) {
-      float* lam_out = (s == 0 && dJdu0) ? dJdu0 : ((lam == g.lamA) ? g.lamB : g.lamA);
-      b.lam = lam;
-      b.p = have_padj ? g.padj : nullptr;
-      b.u = stored ? g.ckpt + (size_t)seg * 2 * NN : g.ustore + (size_t)(s - s0) * 2 * NN;
-      b.lam_out = lam_out;
-      b.step = s;
-      NSGB_CUDA(launch_adjoint_stencil(b, st));
-      if (s > 0) {
-        NSGB_CUDA(poisson_fft(plan->N, fft_launch(plan, w.rhs, w.spec, g.padj), st));
-        have_padj = true;
+  // checkpoint, then run the adjoint steps backwards through them, all but the
+  // last one (s = 0).
+  cudaError_t backward_rest(cudaStream_t st) const {
+    cudaError_t e = cudaSuccess;
+    const RolloutWs& w = g.f;
+    for (int seg = (steps - 1) / every; seg >= 0; --seg) {
+      const int s0 = seg * every, s1 = std::min(steps, s0 + every);
+      const float* rc = g.ckpt + (size_t)seg * 2 * NN;
+      const float* rp = nullptr;
+      for (int s = s0; s < s1 && s1 - s0 > 1 && e == cudaSuccess; ++s) {
+        float* out = ((s - s0) % 2 == 0) ? w.usA : w.usB;
+        e = rollout_step(plan, a, rc, rp, out, w, s, nullptr, g.ustore + (size_t)(s - s0) * 2 * NN, s + 1 < s1, st);
+        rc = out;
+        rp = w.p;
       }
-      lam = lam_out;
+      for (int s = s1 - 1; s >= std::max(s0, 1) && e == cudaSuccess; --s) {
+        e = launch_adjoint_stencil(adjoint_args(s, s0, s1, nullptr), st);
+        if (e == cudaSuccess) e = poisson_fft(plan->N, fft_launch(plan, w.rhs, w.spec, g.padj), st);
+      }
+      if (e != cudaSuccess) break;
     }
+    return e;
   }
-  NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
+};
+
+// Part 0 (forward_rest) or 1 (backward_rest) of a call, as a graph from the
+// second call with the same key on (an optimisation loop, a training loop over
+// changing inputs); one-off calls run eagerly, without the capture's host
+// cost.  Inside a caller's stream capture the launches are simply recorded.
+int grad_part(nsgb_plan* pl, const GradCall& call, int part, const void* ws, cudaStream_t st) {
+  auto enqueue = [&](cudaStream_t s) { return part == 0 ? call.forward_rest(s) : call.backward_rest(s); };
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  NSGB_CUDA(cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone || call.steps < 2) {
+    NSGB_CUDA(enqueue(st));
+    return NSGB_OK;
+  }
+  GradKey key;
+  std::memset(&key, 0, sizeof key);
+  key.ws = ws;
+  key.part = part;
+  key.theta_len = call.theta_len;
+  key.steps = call.steps;
+  key.every = call.every;
+  key.scheme = call.a.scheme;
+  key.c = call.a.c;
+  std::unique_lock<std::mutex> lk(pl->mu);
+  const int t8[8] = {pl->tile_w, pl->tile_h, pl->rows_per_cta, pl->cols_per_cta,
+                     pl->radix_rows, pl->radix_cols, pl->adj_w, pl->adj_h};
+  std::memcpy(key.tiles, t8, sizeof t8);
+  cudaGraphExec_t exec = nullptr;
+  for (auto& e : pl->grad_graphs)
+    if (std::memcmp(&e.first, &key, sizeof key) == 0) exec = e.second;
+  if (!exec) {
+    const bool repeat = std::memcmp(&pl->last_grad[part], &key, sizeof key) == 0;
+    std::memcpy(&pl->last_grad[part], &key, sizeof key);
+    if (!repeat) {
+      lk.unlock();
+      NSGB_CUDA(enqueue(st));
+      return NSGB_OK;
+    }
+    if (!pl->graph_stream) NSGB_CUDA(cudaStreamCreateWithFlags(&pl->graph_stream, cudaStreamNonBlocking));
+    cudaGraph_t graph = nullptr;
+    NSGB_CUDA(cudaStreamBeginCapture(pl->graph_stream, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t ce = enqueue(pl->graph_stream);
+    const cudaError_t ee = cudaStreamEndCapture(pl->graph_stream, &graph);
+    if (ce != cudaSuccess) {
+      if (graph) cudaGraphDestroy(graph);
+      return cuda_fail(ce, "gradient graph capture");
+    }
+    if (ee != cudaSuccess) return cuda_fail(ee, "cudaStreamEndCapture (gradient)");
+    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (ie != cudaSuccess) return cuda_fail(ie, "cudaGraphInstantiate (gradient)");
+    if (pl->grad_graphs.size() >= 8) {
+      cudaGraphExecDestroy(pl->grad_graphs.front().second);
+      pl->grad_graphs.erase(pl->grad_graphs.begin());
+    }
+    pl->grad_graphs.emplace_back(key, exec);
+  }
+  // captured on the plan's private stream, replayed on the caller's
+  NSGB_CUDA(cudaGraphLaunch(exec, st));
   return NSGB_OK;
 }
 }  // namespace
@@ -1460,76 +1510,43 @@ int nsgb_rollout_grad(const nsgb_plan* plan, const nsgb_phys* phys, const float*
   if (int r = check_ws(workspace, ws_bytes, need)) return r;
   cudaStream_t st = (cudaStream_t)stream;
   nsgb_plan* pl = const_cast<nsgb_plan*>(plan);
-  // Inside a caller's stream capture the work is simply recorded.
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  NSGB_CUDA(cudaStreamIsCapturing(st, &cap));
-  if (cap != cudaStreamCaptureStatusNone)
-    return grad_enqueue(plan, phys, u0, theta, theta_len, steps, every, phases, J, u_final, dJdtheta, dJdu0,
-                        workspace, st);  // (a capture is checked when it runs)
-  if (resident_plan(plan, true)) {  // three launches: nothing to gain from a graph
-    const int r = grad_enqueue(plan, phys, u0, theta, theta_len, steps, every, phases, J, u_final, dJdtheta, dJdu0,
-                               workspace, st);
-    return r ? r : finish_call(st);
+  GradCall call(plan, phys, theta_len, steps, every, workspace);
+  const GradWs& g = call.g;
+  const double dx = plan->L / plan->N, jscale = (double)phys->dt * dx * dx;
+  const int nblk = stencil_nblocks(plan->N, call.a.tw, call.a.th);
+  const int adj_nblk = stencil_nblocks(plan->N, call.b.tw, call.b.th);
+
+  if (resident_plan(plan, true)) {
+    call.a.theta = theta;
+    ResidentArgs r = resident_args(plan, call.a, g.f, steps);
+    r.every = every;
+    r.phases = phases;
+    r.u0 = u0;
+    r.u_final = u_final;
+    r.ckpt = g.ckpt;
+    r.ustore = g.ustore;
+    r.lam = g.lamA;
+    r.padj = g.padj;
+    r.gpart = g.gpart;
+    r.dJdu0 = dJdu0;
+    NSGB_CUDA(launch_resident(plan->N, r, st));
+    if (phases & NSGB_GRAD_FORWARD) NSGB_CUDA(launch_jreduce(g.f.jpart, nblk, steps, g.f.jsteps, J, jscale, st));
+    if (phases & NSGB_GRAD_BACKWARD) NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
+    return finish_call(st);
   }
-  GradKey key;
-  std::memset(&key, 0, sizeof key);
-  key.ws = workspace;
-  key.u0 = u0;
-  key.theta = theta;
-  key.J = J;
-  key.u_final = u_final;
-  key.dJdtheta = dJdtheta;
-  key.dJdu0 = dJdu0;
-  key.theta_len = theta_len;
-  key.steps = steps;
-  key.every = every;
-  key.phases = phases;
-  key.scheme = phys->scheme;
-  {
-    StencilArgs a = stencil_args(plan, phys);
-    key.c = a.c;
+
+  NSGB_CUDA(cudaMemcpyAsync(g.f.theta, theta, theta_len * sizeof(float), cudaMemcpyDeviceToDevice, st));
+  if (phases & NSGB_GRAD_FORWARD) {
+    NSGB_CUDA(call.forward_step(0, u0, st));
+    if (int r = grad_part(pl, call, 0, workspace, st)) return r;
+    if (u_final) NSGB_CUDA(launch_project(call.last_us(), g.f.p, u_final, call.a.c, st));
+    NSGB_CUDA(launch_jreduce(g.f.jpart, nblk, steps, g.f.jsteps, J, jscale, st));
   }
-  std::unique_lock<std::mutex> lk(pl->mu);
-  const int t8[8] = {pl->tile_w, pl->tile_h, pl->rows_per_cta, pl->cols_per_cta,
-                     pl->radix_rows, pl->radix_cols, pl->adj_w, pl->adj_h};
-  std::memcpy(key.tiles, t8, sizeof t8);
-  cudaGraphExec_t exec = nullptr;
-  for (auto& e : pl->grad_graphs)
-    if (std::memcmp(&e.first, &key, sizeof key) == 0) exec = e.second;
-  if (!exec) {
-    // A call is captured as a graph the second time it is made with the same
-    // arguments (an optimisation loop, repeated timing); one-off calls run
-    // eagerly, without the capture's host cost.
-    const bool repeat = std::memcmp(&pl->last_grad, &key, sizeof key) == 0;
-    std::memcpy(&pl->last_grad, &key, sizeof key);
-    if (!repeat) {
-      lk.unlock();
-      const int r = grad_enqueue(plan, phys, u0, theta, theta_len, steps, every, phases, J, u_final, dJdtheta,
-                                 dJdu0, workspace, st);
-      return r ? r : finish_call(st);
-    }
-    if (!pl->graph_stream) NSGB_CUDA(cudaStreamCreateWithFlags(&pl->graph_stream, cudaStreamNonBlocking));
-    cudaGraph_t graph = nullptr;
-    NSGB_CUDA(cudaStreamBeginCapture(pl->graph_stream, cudaStreamCaptureModeThreadLocal));
-    const int r = grad_enqueue(plan, phys, u0, theta, theta_len, steps, every, phases, J, u_final, dJdtheta,
-                               dJdu0, workspace, pl->graph_stream);
-    const cudaError_t ee = cudaStreamEndCapture(pl->graph_stream, &graph);
-    if (r != NSGB_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return r;
-    }
-    if (ee != cudaSuccess) return cuda_fail(ee, "cudaStreamEndCapture (gradient)");
-    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ie != cudaSuccess) return cuda_fail(ie, "cudaGraphInstantiate (gradient)");
-    if (pl->grad_graphs.size() >= 4) {
-      cudaGraphExecDestroy(pl->grad_graphs.front().second);
-      pl->grad_graphs.erase(pl->grad_graphs.begin());
-    }
-    pl->grad_graphs.emplace_back(key, exec);
+  if (phases & NSGB_GRAD_BACKWARD) {
+    if (int r = grad_part(pl, call, 1, workspace, st)) return r;
+    NSGB_CUDA(launch_adjoint_stencil(call.adjoint_args(0, 0, std::min(steps, every), dJdu0), st));
+    NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
   }
-  // captured on the plan's private stream, replayed on the caller's
-  NSGB_CUDA(cudaGraphLaunch(exec, st));
   return finish_call(st);
 }
 
@@ -1547,7 +1564,7 @@ struct GradOp {
 };
 inline int grad_seg_ops(int len) { return len == 1 ? 1 : 2 * len; }
 
-// The operations in the order grad_enqueue issues them: `steps` forward steps,
+// The operations in the order nsgb_rollout_grad issues them: `steps` forward steps,
 // then per checkpoint segment, last first, its recomputed steps (none for a
 // one-step segment, whose state is its checkpoint) and its adjoint steps.
 int grad_ops_total(int steps, int every) {
@@ -1687,7 +1704,7 @@ StencilArgs grad_fwd_args(const nsgb_grad_member& m, const GradMemberCtx& c, con
   return x;
 }
 
-// Arguments of adjoint step o (grad_enqueue's lambda ping-pong: the adjoint
+// Arguments of adjoint step o (GradCall's lambda ping-pong: the adjoint
 // step b = steps - 1 - s writes lamA for even b, lamB for odd b).
 AdjointArgs grad_adj_args(const nsgb_grad_member& m, const GradMemberCtx& c, const GradOp& o) {
   AdjointArgs x = c.b;
