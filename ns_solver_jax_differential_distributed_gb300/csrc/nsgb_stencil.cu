@@ -22,17 +22,34 @@
 
 namespace nsgb {
 
+// Tiles at least 64 wide use the body with four cells per thread (a block of
+// TW/4 x TH threads in one dimension), narrower ones a block of 32 x 8.
+template <int TW>
+constexpr bool wide_tile() {
+  return TW >= 64;
+}
+template <int TW, int TH>
+constexpr int tile_threads() {
+  return wide_tile<TW>() ? TW / 4 * TH : 256;
+}
+
 template <int SCHEME, int MODE, int TW, int TH>
-__global__ void __launch_bounds__(256) k_stencil(const StencilArgs a) {
-  stencil_body<SCHEME, MODE, TW, TH>(a, 0, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
+__global__ void __launch_bounds__((tile_threads<TW, TH>())) k_stencil(const StencilArgs a) {
+  if constexpr (wide_tile<TW>())
+    stencil4_body<SCHEME, MODE, TW, TH>(a, 0, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
+  else
+    stencil_body<SCHEME, MODE, TW, TH>(a, 0, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
 }
 
 // Ensemble variant: blockIdx.z selects the solve, `variant` its argument set.
 template <int SCHEME, int TW, int TH>
-__global__ void __launch_bounds__(256) k_stencil_batch(const SolveDev* __restrict__ solves, int variant,
-                                                      int step_off) {
-  stencil_body<SCHEME, MODE_ROLLOUT, TW, TH>(solves[blockIdx.z].st[variant], step_off, blockIdx.x, blockIdx.y,
-                                             gridDim.x, gridDim.y);
+__global__ void __launch_bounds__((tile_threads<TW, TH>())) k_stencil_batch(const SolveDev* __restrict__ solves,
+                                                                          int variant, int step_off) {
+  const StencilArgs& a = solves[blockIdx.z].st[variant];
+  if constexpr (wide_tile<TW>())
+    stencil4_body<SCHEME, MODE_ROLLOUT, TW, TH>(a, step_off, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
+  else
+    stencil_body<SCHEME, MODE_ROLLOUT, TW, TH>(a, step_off, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
 }
 
 // ------------------------------------------------------- row streaming --
@@ -406,7 +423,14 @@ bool stencil_tile_supported(int tw, int th) {
 
 template <int TW, int TH>
 static constexpr size_t stencil_smem() {
-  return StencilSmem<TW, TH>::FLOATS * sizeof(float);
+  if constexpr (wide_tile<TW>())
+    return Stencil4Smem<TW, TH>::FLOATS * sizeof(float);
+  else
+    return StencilSmem<TW, TH>::FLOATS * sizeof(float);
+}
+template <int TW, int TH>
+static dim3 tile_block() {
+  return wide_tile<TW>() ? dim3(tile_threads<TW, TH>()) : dim3(32, 8);
 }
 
 template <int SCHEME, int MODE, int TW, int TH>
@@ -414,7 +438,7 @@ static cudaError_t launch_stencil_t(const StencilArgs& a, cudaStream_t st) {
   const cudaError_t e = raise_smem_limit(k_stencil<SCHEME, MODE, TW, TH>);
   if (e != cudaSuccess) return e;
   const dim3 grid(a.c.N / TW, a.c.N / TH);
-  k_stencil<SCHEME, MODE, TW, TH><<<grid, dim3(32, 8), stencil_smem<TW, TH>(), st>>>(a);
+  k_stencil<SCHEME, MODE, TW, TH><<<grid, tile_block<TW, TH>(), stencil_smem<TW, TH>(), st>>>(a);
   return cudaGetLastError();
 }
 
@@ -424,7 +448,7 @@ static cudaError_t launch_stencil_batch_t(const SolveDev* solves, int count, int
   const cudaError_t e = raise_smem_limit(k_stencil_batch<SCHEME, TW, TH>);
   if (e != cudaSuccess) return e;
   const dim3 grid(N / TW, N / TH, count);
-  k_stencil_batch<SCHEME, TW, TH><<<grid, dim3(32, 8), stencil_smem<TW, TH>(), st>>>(solves, variant,
+  k_stencil_batch<SCHEME, TW, TH><<<grid, tile_block<TW, TH>(), stencil_smem<TW, TH>(), st>>>(solves, variant,
                                                                                    step_off);
   return cudaGetLastError();
 }
