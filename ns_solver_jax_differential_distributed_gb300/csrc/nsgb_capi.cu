@@ -1193,6 +1193,15 @@ int nsgb_step(const nsgb_plan* plan, const nsgb_phys* phys, const float* u, cons
   a.step_fixed = 0;
   a.t_from_step = 0;
   a.t_fixed = t;
+  if (resident_plan(plan, false)) {  // the five launches below in one
+    ResidentArgs r = resident_args(plan, a, w, 1);
+    r.t_from_step = 0;
+    r.t_fixed = t;
+    r.u0 = u;
+    r.u_final = u_out;
+    NSGB_CUDA(launch_resident(plan->N, r, st));
+    return finish_call(st);
+  }
   NSGB_CUDA(launch_stencil(a, MODE_ROLLOUT, st));
   NSGB_CUDA(poisson_fft(plan->N, fft_launch(plan, w.rhs, w.spec, w.p), st));
   NSGB_CUDA(launch_project(w.usA, w.p, u_out, a.c, st));

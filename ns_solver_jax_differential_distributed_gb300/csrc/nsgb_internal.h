@@ -198,6 +198,8 @@ struct ResidentArgs {
   int theta_len = 2;
   int steps = 0, every = 1;
   int phases = 1;              // NSGB_GRAD_FORWARD | NSGB_GRAD_BACKWARD
+  int t_from_step = 1;         // forcing time step * dt, or t_fixed (a single step)
+  float t_fixed = 0.f;
   const float* u0 = nullptr;   // forward
   float* jpart = nullptr;      // objective partials, [step][tile]
   float* u_final = nullptr;    // optional

@@ -186,7 +186,7 @@ struct Solve {
   // step, by the last two warps, which no transform uses.
   __device__ __forceinline__ void forcing(int step, bool adjoint) {
     if (warp < NW - 2) return;
-    const float t = fmul((float)step, c.dt);
+    const float t = a.t_from_step ? fmul((float)step, c.dt) : a.t_fixed;
     const float tA = gldg(a.theta), tB = gldg(a.theta + 1);
     const ForcingRow fr = forcing_time(tA, tB, t, c);
     if (warp == NW - 1) {

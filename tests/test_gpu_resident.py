@@ -79,6 +79,15 @@ def test_gradients_equal_tiled_and_batched(nat, N, scheme, steps, every):
     assert torch.equal(J, Jb) and torch.equal(g, gbt) and torch.equal(du, gb.du0(sid)), (g, gbt)
 
 
+@pytest.mark.parametrize("N", SIZES)
+def test_single_steps_equal_the_tiled_step(nat, N):
+    u0, th = _inputs(N, 2)
+    for sch in (0, 1):
+        def step():
+            return nat.op_step(u0, th, 0.37, L, NU, DT, sch, 0.5, 0.1, 1.0)
+        assert torch.equal(step(), _tiled(nat, N, step))
+
+
 def test_phases_one_by_one(nat):
     """Forward then backward (a differentiable rollout) equals one call."""
     u0, th = _inputs(64)
