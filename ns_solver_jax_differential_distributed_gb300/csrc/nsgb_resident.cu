@@ -85,6 +85,11 @@ __device__ __forceinline__ unsigned cta_rank() {
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
+// The CTAs of a cluster are placed together but need not have begun together:
+// no store to another CTA's shared memory before it runs (arrive when a CTA
+// begins, wait before its first such store), none after it has ended.
+__device__ __forceinline__ void cluster_begin() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_begun() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ uint32_t remote(uint32_t local, unsigned rank) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
@@ -490,6 +495,7 @@ struct Solve {
   }
 
   __device__ __forceinline__ void run() {
+    cluster_begin();
     bool fready = false;  // the next operation's forcing is in shared memory
     auto need_forcing = [&](int step, bool adj) {
       if (!fready) forcing(step, adj);
@@ -498,6 +504,7 @@ struct Solve {
     if (a.phases & NSGB_GRAD_FORWARD) {
       load<R + 4, 2>(A, a.u0, r0 - 2);
       need_forcing(0, false);
+      cluster_begun();
       for (int s = 0; s < a.steps; ++s) {
         float* ck = (a.ckpt && s % a.every == 0) ? a.ckpt + (size_t)(s / a.every) * 2 * N * N : nullptr;
         forward(s > 0, ck);
@@ -519,6 +526,7 @@ struct Solve {
       if (!(a.phases & NSGB_GRAD_BACKWARD)) return;
       const int nseg = (a.steps + a.every - 1) / a.every;
       bool have_lam = false, have_p = false, uready = false;
+      if (!(a.phases & NSGB_GRAD_FORWARD)) cluster_begun();
       __syncthreads();
       for (int seg = nseg - 1; seg >= 0; --seg) {
         const int s0 = seg * a.every, s1 = min(a.steps, s0 + a.every);
@@ -568,6 +576,7 @@ struct Solve {
             __syncthreads();
             combine<kTheta>(0, !have_lam);
             if (a.dJdu0) store_own(B, a.dJdu0);
+            cluster_barrier();  // the neighbours' halo rows have arrived: CTAs may end
           }
           have_lam = true;
           swap();
