@@ -188,7 +188,7 @@ cudaError_t launch_gsum(const double* gpart, int nblk, int theta_len, float* dJ,
 // A rollout or a gradient of a small grid in one cluster launch
 // (nsgb_resident.cu); the pointers are those of the batched path, which it
 // replaces value for value at 32 x 8 tiles.
-struct ResidentArgs {
+struct alignas(16) ResidentArgs {
   StepConsts c;
   int scheme = 0;
   const float2* tw = nullptr;  // twiddles of the resident radix
@@ -197,22 +197,30 @@ struct ResidentArgs {
   const float* theta = nullptr;
   int theta_len = 2;
   int steps = 0, every = 1;
-  int phases = 1;              // NSGB_GRAD_FORWARD | NSGB_GRAD_BACKWARD
+  // Operations [op0, op1) of the schedule of a gradient solve (grad_op): the
+  // forward steps, then per checkpoint segment, last first, its recomputed and
+  // its adjoint steps.  A launch that does not start at the first operation
+  // takes up the state the previous one left in the buffers below, which are
+  // those of the batched gradients, step for step.
+  int op0 = 0, op1 = 0;
   int t_from_step = 1;         // forcing time step * dt, or t_fixed (a single step)
   float t_fixed = 0.f;
-  const float* u0 = nullptr;   // forward
+  const float* u0 = nullptr;
   float* jpart = nullptr;      // objective partials, [step][tile]
   float* u_final = nullptr;    // optional
   float* ckpt = nullptr;       // checkpoints every `every` steps (nullptr: a plain rollout)
   float* ustore = nullptr;     // a segment's states
-  float* lam = nullptr;        // lambda and its pressure while a segment is recomputed
-  float* padj = nullptr;
+  float *usA = nullptr, *usB = nullptr, *p = nullptr;         // u* (by parity) and pressure
+  float *lamA = nullptr, *lamB = nullptr, *padj = nullptr;    // lambda (by parity) and its pressure
   double* gpart = nullptr;     // theta sensitivities, [tile][3]
   float* dJdu0 = nullptr;      // optional
 };
 int resident_radix(int N);        // radix of its transforms, 0: no instance for N
-bool resident_available(int N);   // the current device can launch its clusters
 cudaError_t launch_resident(int N, const ResidentArgs& a, cudaStream_t st);
+// Gradient solves of one scheme, one cluster each, in one launch: tab is a
+// device table of their arguments.
+cudaError_t launch_resident_batch(int N, int scheme, const ResidentArgs* tab, int count, cudaStream_t st);
+int resident_clusters(int N);     // clusters the current device runs at once (0: no instance, or none); call first
 
 // ------------------------------------------------------------- optimiser --
 // Constants of one optimiser update, float32 as the library rounds them;

@@ -1,20 +1,19 @@
 // Resident solves of small grids: a whole rollout, or a whole gradient (forward
-// steps, recomputed segments and adjoint steps), in one launch of one thread
-// block cluster.
+// steps, recomputed segments and adjoint steps), or any stretch of a batched
+// gradient's operations, in one launch of one thread block cluster per solve.
 //
 // Up to N = 128 a step's four launches cost more than their work.  Here C CTAs,
 // one cluster, own R = N / C rows each and keep the state (u* or lambda, the
 // pressure, and the spectrum's pieces) in shared memory for all steps.
 // Measured per step against four launches in a graph: N = 32 3.1 / 7.8 us, 64
-// 3.2 / 8.0, 128 4.7 / 8.9; with the gradient, every state kept, 8.2 / 15.7, 8.2 /
-// 16.0, 11.3 / 17.8.  At N = 256 sixteen CTAs have too many cells each (10.0 / 10.4
+// 3.1 / 8.0, 128 4.8 / 8.9; with the gradient, every state kept, 7.7 / 15.8, 7.7 /
+// 15.9, 11.3 / 17.9.  At N = 256 sixteen CTAs have too many cells each (10.0 / 10.4
 // and 24 / 21 us), so the four launches stay.  What bounds a step is latency:
 // three cluster barriers of about 0.35 us and four transforms of a few warps
 // of about 0.5 us; so transforms are of radix 8 (radix 16 on half the threads
 // took 9.4 us per step at N = 128), cells go four to a thread, and the
 // objective and theta sums run in the warps that the row transforms leave
-// idle.  A
-// step is three phases between cluster barriers:
+// idle.  A step is three phases between cluster barriers:
 //   1. stencil of the own rows (halo rows are kept beside them), right-hand
 //      side, forward row transforms, split into the two rows' half spectra and
 //      sent to the CTAs that own the columns (distributed shared memory);
@@ -30,6 +29,8 @@
 // radix, objective and theta partials summed per 32 x 8 tile in the same
 // order, so a resident solve, an ensemble member and a batched gradient give
 // the same bits.
+#include <type_traits>
+
 #include "nsgb_adjoint_cell.cuh"
 #include "nsgb_fft_bodies.cuh"
 #include "nsgb_internal.h"
@@ -494,98 +495,196 @@ struct Solve {
     __syncthreads();
   }
 
+  // ---- the schedule (nsgb_capi.cu: grad_op) ----
+  enum Kind { kFwd, kRec, kAdj };
+  struct Op {
+    int kind, s, s0, s1;  // step; its segment [s0, s1) (recomputed and adjoint steps)
+  };
+  __device__ __forceinline__ Op segment(int seg) const {  // the first operation of a segment
+    const int s0 = seg * a.every, s1 = min(a.steps, s0 + a.every);
+    return {s1 - s0 > 1 ? kRec : kAdj, s0, s0, s1};  // a one-step segment's state is its checkpoint
+  }
+  __device__ __forceinline__ Op op_at(int k) const {
+    if (k < a.steps) return {kFwd, k, 0, 0};
+    k -= a.steps;
+    for (int seg = (a.steps - 1) / a.every;; --seg) {
+      Op o = segment(seg);
+      const int len = o.s1 - o.s0, n = len > 1 ? 2 * len : 1;
+      if (k >= n) {
+        k -= n;
+        continue;
+      }
+      if (len > 1 && k < len)
+        o.s = o.s0 + k;
+      else
+        o.kind = kAdj, o.s = o.s1 - 1 - (len > 1 ? k - len : k);
+      return o;
+    }
+  }
+  __device__ __forceinline__ Op next_op(Op o) const {
+    if (o.kind == kFwd) {
+      if (++o.s < a.steps) return o;
+      return segment((a.steps - 1) / a.every);
+    }
+    if (o.kind == kRec) {
+      if (++o.s == o.s1) o.kind = kAdj, --o.s;
+      return o;
+    }
+    if (--o.s >= o.s0) return o;
+    return segment(o.s0 / a.every - 1);
+  }
+  // The buffers of a step's results, by parity (grad_fwd_args, grad_adj_args).
+  __device__ __forceinline__ float* us_of(const Op& o) const {
+    return (o.s - (o.kind == kRec ? o.s0 : 0)) % 2 == 0 ? a.usA : a.usB;
+  }
+  __device__ __forceinline__ float* lam_of(int s) const { return (a.steps - 1 - s) % 2 == 0 ? a.lamA : a.lamB; }
+  __device__ __forceinline__ const float* u_of(const Op& o) const {  // u_s of an adjoint step
+    return o.s1 - o.s0 == 1 ? a.ckpt + (size_t)(o.s0 / a.every) * 2 * N * N
+                            : a.ustore + (size_t)(o.s - o.s0) * 2 * N * N;
+  }
+
+  // The field in A and the pressure to or from global memory.
+  __device__ __forceinline__ void save(float* f, float* p) const {
+    store_own(A, f);
+    const float* P = sm + L::P_OFF;
+    for (int e = tid; e < R * N; e += NT) gst(p + (size_t)r0 * N + e, P[3 * N + e]);
+  }
+  __device__ __forceinline__ void restore(const float* f, const float* p) {
+    load<R + 4, 2>(A, f, r0 - 2);
+    load<R + 6, 1>(sm + L::P_OFF, p, r0 - 3);
+  }
+
+  // Makes the state of operation o present; `before`: the kind of the operation
+  // this launch ran before it, -1 if none.  The caller's next barrier publishes
+  // it within the CTA.
+  __device__ __forceinline__ void enter(const Op& o, int before, int prev_s) {
+    if (o.kind == kFwd) {
+      if (o.s == 0)
+        load<R + 4, 2>(A, a.u0, r0 - 2);
+      else
+        restore(us_of({kFwd, o.s - 1, 0, 0}), a.p);
+    } else if (o.kind == kRec) {
+      if (before == kAdj) {  // lambda and its pressure wait in global memory
+        save(lam_of(prev_s), a.padj);
+        cluster_barrier();
+      }
+      if (o.s == o.s0)
+        load<R + 4, 2>(A, a.ckpt + (size_t)(o.s0 / a.every) * 2 * N * N, r0 - 2);
+      else
+        restore(us_of({kRec, o.s - 1, o.s0, o.s1}), a.p);
+    } else if (o.s == a.steps - 1) {
+      for (int e = tid; e < 2 * UP; e += NT) A[e] = 0.f;
+    } else if (before != kAdj) {
+      restore(lam_of(o.s + 1), a.padj);
+    }
+    if (GRAD && o.kind == kAdj) prefetch_u(u_of(o));
+    forcing(o.s, o.kind == kAdj);
+  }
+
+  __device__ __forceinline__ void project_final() const {
+    const float* P = sm + L::P_OFF;
+    for (int e = tid; e < R * N; e += NT) {
+      const int r = e / N, cc = e % N, o = (r + 2) * N + cc;
+      const float* p0 = P + (r + 3) * N;
+      gst(a.u_final + (size_t)r0 * N + e, fused_proj(A[o], p0[N + cc], p0[cc - N], c.cP));
+      gst(a.u_final + (size_t)N * N + (size_t)r0 * N + e,
+          fused_proj(A[UP + o], p0[(cc + 1) & M], p0[(cc - 1) & M], c.cP));
+    }
+  }
+
+  // Operations [op0, op1), in runs of one kind (one loop each: a loop over
+  // operations of every kind cost 0.4 us per step).
   __device__ __forceinline__ void run() {
+    if (a.op0 >= a.op1) return;
     cluster_begin();
-    bool fready = false;  // the next operation's forcing is in shared memory
-    auto need_forcing = [&](int step, bool adj) {
-      if (!fready) forcing(step, adj);
-      __syncthreads();
-    };
-    if (a.phases & NSGB_GRAD_FORWARD) {
-      load<R + 4, 2>(A, a.u0, r0 - 2);
-      need_forcing(0, false);
-      cluster_begun();
-      for (int s = 0; s < a.steps; ++s) {
-        float* ck = (a.ckpt && s % a.every == 0) ? a.ckpt + (size_t)(s / a.every) * 2 * N * N : nullptr;
-        forward(s > 0, ck);
-        poisson<kObjective>(s, false, s + 1 < a.steps ? s + 1 : -1, nullptr);
+    constexpr int NG = (R / kTileH) * S * 3;  // the CTA's running theta sums
+    double* acc = reinterpret_cast<double*>(sm + L::GA_OFF);
+    Op o = op_at(a.op0);
+    if constexpr (GRAD) {
+      // adjoint steps done by earlier launches
+      if (o.kind != kFwd && a.steps - (o.kind == kRec ? o.s1 : o.s + 1) > 0)
+        for (int e = tid; e < NG; e += NT) acc[e] = gld(a.gpart + (size_t)(r0 / kTileH) * S * 3 + e);
+    }
+    enter(o, -1, 0);
+    cluster_begun();
+    __syncthreads();
+    int left = a.op1 - a.op0;
+    if (o.kind == kFwd) {
+      const int s1 = min(a.steps, o.s + left);
+      left -= s1 - o.s;
+      for (int s = o.s; s < s1; ++s) {
+        forward(s > 0, (GRAD && s % a.every == 0) ? a.ckpt + (size_t)(s / a.every) * 2 * N * N : nullptr);
+        poisson<kObjective>(s, false, s + 1 < s1 ? s + 1 : -1, nullptr);
         swap();
       }
-      if (a.u_final) {
-        const float* P = sm + L::P_OFF;
-        for (int e = tid; e < R * N; e += NT) {
-          const int r = e / N, cc = e % N, o = (r + 2) * N + cc;
-          const float* p0 = P + (r + 3) * N;
-          gst(a.u_final + (size_t)r0 * N + e, fused_proj(A[o], p0[N + cc], p0[cc - N], c.cP));
-          gst(a.u_final + (size_t)N * N + (size_t)r0 * N + e,
-              fused_proj(A[UP + o], p0[(cc + 1) & M], p0[(cc - 1) & M], c.cP));
-        }
+      o.s = s1 - 1;
+      if (s1 < a.steps) {
+        if constexpr (GRAD) save(us_of(o), a.p);
+        return;
       }
+      if (a.u_final) project_final();
     }
     if constexpr (GRAD) {
-      if (!(a.phases & NSGB_GRAD_BACKWARD)) return;
-      const int nseg = (a.steps + a.every - 1) / a.every;
-      bool have_lam = false, have_p = false, uready = false;
-      if (!(a.phases & NSGB_GRAD_FORWARD)) cluster_begun();
-      __syncthreads();
-      for (int seg = nseg - 1; seg >= 0; --seg) {
-        const int s0 = seg * a.every, s1 = min(a.steps, s0 + a.every);
-        const float* ck = a.ckpt + (size_t)seg * 2 * N * N;
-        const bool stored = s1 - s0 == 1;  // a one-step segment's state is its checkpoint
-        if (!stored) {
-          if (have_lam) {  // lambda and its pressure wait in global memory
-            store_own(A, a.lam);
-            const float* P = sm + L::P_OFF;
-            for (int e = tid; e < R * N; e += NT) gst(a.padj + (size_t)r0 * N + e, P[3 * N + e]);
-            cluster_barrier();
-          }
-          load<R + 4, 2>(A, ck, r0 - 2);
-          fready = false;
-          need_forcing(s0, false);
-          for (int s = s0; s < s1; ++s) {
-            forward(s > s0, a.ustore + (size_t)(s - s0) * 2 * N * N);
-            if (s + 1 < s1)
-              poisson<kNone>(0, false, s + 1, nullptr);
+      if (o.kind == kFwd) {
+        if (!left) return;
+        const Op nx = next_op(o);
+        __syncthreads();  // the state is not overwritten under a reader
+        enter(nx, kFwd, o.s);
+        __syncthreads();
+        o = nx;
+      }
+      for (;;) {
+        if (o.kind == kRec) {
+          const int s1 = min(o.s1, o.s + left);
+          left -= s1 - o.s;
+          for (int s = o.s; s < s1; ++s) {
+            forward(s > o.s0, a.ustore + (size_t)(s - o.s0) * 2 * N * N);
+            if (s + 1 < o.s1)
+              poisson<kNone>(0, false, s + 1 < s1 ? s + 1 : -1, nullptr);
             else
               cluster_barrier();  // the neighbours' states are written
             swap();
           }
-          if (have_lam) {
-            load<R + 4, 2>(A, a.lam, r0 - 2);
-            load<R + 6, 1>(sm + L::P_OFF, a.padj, r0 - 3);
-          }
-          fready = false;
-        }
-        if (!uready) prefetch_u(stored ? ck : a.ustore + (size_t)(s1 - 1 - s0) * 2 * N * N);
-        for (int s = s1 - 1; s >= s0; --s) {
-          if (!have_lam)
-            for (int e = tid; e < 2 * UP; e += NT) A[e] = 0.f;
-          asm volatile("cp.async.wait_all;" ::: "memory");
-          need_forcing(s, true);
-          adjoint(have_p);
-          // the next adjoint step's state arrives during the Poisson solve
-          uready = s > s0 || (s > 0 && a.every == 1);
-          const float* u_next = !uready ? nullptr
-                                : s > s0 ? a.ustore + (size_t)(s - 1 - s0) * 2 * N * N
-                                         : a.ckpt + (size_t)(s - 1) * 2 * N * N;
-          if (s > 0) {
-            poisson<kTheta>(0, !have_lam, s - 1, u_next);
-            have_p = fready = true;
-          } else {
-            sums<kTheta>(0);
+          o.s = s1 - 1;
+        } else {
+          // states kept one by one: one run through all segments
+          const int low = max(o.s + 1 - left, a.every == 1 ? 0 : o.s0);
+          left -= o.s + 1 - low;
+          const float* u = u_of(o);
+          for (int s = o.s; s >= low; --s) {
+            const bool first = s == a.steps - 1;
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
-            combine<kTheta>(0, !have_lam);
-            if (a.dJdu0) store_own(B, a.dJdu0);
-            cluster_barrier();  // the neighbours' halo rows have arrived: CTAs may end
+            adjoint(!first);
+            u -= 2 * N * N;
+            if (s > 0) {
+              // the next adjoint step's state arrives during the Poisson solve
+              poisson<kTheta>(0, first, s > low ? s - 1 : -1, s > low ? u : nullptr);
+            } else {
+              sums<kTheta>(0);
+              __syncthreads();
+              combine<kTheta>(0, first);
+              if (a.dJdu0) store_own(B, a.dJdu0);
+              cluster_barrier();  // the neighbours' halo rows have arrived: CTAs may end
+            }
+            swap();
           }
-          have_lam = true;
-          swap();
+          o.s = low;
+          if (a.every == 1) o.s0 = low;
         }
+        if (!left) break;
+        const Op nx = next_op(o);
+        __syncthreads();  // the state is not overwritten under a reader
+        enter(nx, o.kind, o.s);
+        __syncthreads();
+        o = nx;
       }
+      // what the next launch takes up
+      if (o.kind == kRec && o.s + 1 < o.s1) save(us_of(o), a.p);
+      if (o.kind == kAdj && o.s > 0) save(lam_of(o.s), a.padj);
       __syncthreads();
-      const double* acc = reinterpret_cast<const double*>(sm + L::GA_OFF);
-      for (int e = tid; e < (R / kTileH) * S * 3; e += NT)
-        gst(a.gpart + (size_t)(r0 / kTileH) * S * 3 + e, acc[e]);
+      if (o.kind == kAdj || o.s1 < a.steps)
+        for (int e = tid; e < NG; e += NT) gst(a.gpart + (size_t)(r0 / kTileH) * S * 3 + e, acc[e]);
     }
   }
 };
@@ -597,6 +696,19 @@ __global__ void __launch_bounds__(Lay<N, R, E>::NT, 1) k_resident(const Resident
   s.run();
 }
 
+// Gradients of several solves: cluster blockIdx.x / C takes the solve's entry.
+template <int N, int R, int E, int SCHEME>
+__global__ void __launch_bounds__(Lay<N, R, E>::NT, 1) k_resident_batch(const ResidentArgs* __restrict__ tab) {
+  extern __shared__ __align__(16) float sm_res[];
+  static_assert(std::is_trivially_copyable<ResidentArgs>::value && sizeof(ResidentArgs) % 16 == 0, "table entries");
+  __shared__ uint4 raw[sizeof(ResidentArgs) / 16];
+  const uint4* src = reinterpret_cast<const uint4*>(tab + blockIdx.x / Lay<N, R, E>::C);
+  for (int e = threadIdx.x; e < (int)(sizeof(ResidentArgs) / 16); e += Lay<N, R, E>::NT) raw[e] = gld(src + e);
+  __syncthreads();
+  Solve<N, R, E, SCHEME, true> s(*reinterpret_cast<const ResidentArgs*>(raw), sm_res);
+  s.run();
+}
+
 }  // namespace res
 
 // Rows per CTA and radix of the resident kernel's instances.
@@ -604,49 +716,50 @@ __global__ void __launch_bounds__(Lay<N, R, E>::NT, 1) k_resident(const Resident
 #define NSGB_RESIDENT(X) X(32, 16, 8) X(64, 8, 8) X(128, 8, 8)
 #endif
 
-template <int N, int R, int E, int SCHEME, bool GRAD>
-static cudaError_t launch_resident_t(const ResidentArgs& a, bool probe, cudaStream_t st) {
-  using L = res::Lay<N, R, E>;
-  auto kernel = res::k_resident<N, R, E, SCHEME, GRAD>;
-  cudaError_t e = raise_smem_limit(kernel);
-  if (e != cudaSuccess) return e;
-  if (probe && L::C > 8) {  // once per device: every launch follows a probe
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
+// Configuration of `count` clusters of an instance; attr outlives it.
+template <class L>
+static cudaLaunchConfig_t cluster_config(bool grad, int count, cudaLaunchAttribute* attr, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(L::C);
+  cfg.gridDim = dim3(L::C * count);
   cfg.blockDim = dim3(L::NT);
-  cfg.dynamicSmemBytes = sizeof(float) * (GRAD ? L::GRAD : L::FWD);
+  cfg.dynamicSmemBytes = sizeof(float) * (grad ? L::GRAD : L::FWD);
   cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = L::C;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = L::C;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (probe) {
-    int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-    return e != cudaSuccess ? e : n < 1 ? cudaErrorInvalidConfiguration : cudaSuccess;
-  }
-  return cudaLaunchKernelEx(&cfg, kernel, a);
+  return cfg;
 }
 
-static cudaError_t resident_dispatch(int N, const ResidentArgs& a, bool grad, bool probe, cudaStream_t st) {
-  const bool up = a.scheme == NSGB_SCHEME_UPWIND;
-#define NSGB_RESIDENT_CASE(NN, R, E)                                                                      \
-  if (N == NN) {                                                                                          \
-    if (grad)                                                                                             \
-      return up ? launch_resident_t<NN, R, E, NSGB_SCHEME_UPWIND, true>(a, probe, st)                     \
-                : launch_resident_t<NN, R, E, NSGB_SCHEME_CENTRAL, true>(a, probe, st);                   \
-    return up ? launch_resident_t<NN, R, E, NSGB_SCHEME_UPWIND, false>(a, probe, st)                      \
-              : launch_resident_t<NN, R, E, NSGB_SCHEME_CENTRAL, false>(a, probe, st);                    \
+// Prepares a kernel for its clusters and asks how many of them the device runs
+// at once (0: none).
+template <class L, class K>
+static int probe_clusters(K* kernel, bool grad) {
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config<L>(grad, 1, &attr, nullptr);
+  int n = 0;
+  if (raise_smem_limit(kernel) != cudaSuccess ||
+      (L::C > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
   }
-  NSGB_RESIDENT(NSGB_RESIDENT_CASE)
-#undef NSGB_RESIDENT_CASE
-  return cudaErrorInvalidValue;
+  return n;
+}
+
+template <int N, int R, int E, int SCHEME, bool GRAD>
+static cudaError_t launch_resident_t(const ResidentArgs& a, cudaStream_t st) {
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config<res::Lay<N, R, E>>(GRAD, 1, &attr, st);
+  return cudaLaunchKernelEx(&cfg, res::k_resident<N, R, E, SCHEME, GRAD>, a);
+}
+template <int N, int R, int E, int SCHEME>
+static cudaError_t launch_resident_batch_t(const ResidentArgs* tab, int count, cudaStream_t st) {
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config<res::Lay<N, R, E>>(true, count, &attr, st);
+  return cudaLaunchKernelEx(&cfg, res::k_resident_batch<N, R, E, SCHEME>, tab);
 }
 
 int resident_radix(int N) {
@@ -656,21 +769,50 @@ int resident_radix(int N) {
   return 0;
 }
 
-bool resident_available(int N) {
-  for (int scheme : {NSGB_SCHEME_CENTRAL, NSGB_SCHEME_UPWIND})
-    for (bool grad : {false, true}) {
-      ResidentArgs a;
-      a.scheme = scheme;
-      if (resident_dispatch(N, a, grad, true, nullptr) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-      }
-    }
-  return true;
+template <int N, int R, int E, int SCHEME>
+static int probe_instances() {
+  using L = res::Lay<N, R, E>;
+  const int f = probe_clusters<L>(res::k_resident<N, R, E, SCHEME, false>, false);
+  const int g = probe_clusters<L>(res::k_resident<N, R, E, SCHEME, true>, true);
+  const int b = probe_clusters<L>(res::k_resident_batch<N, R, E, SCHEME>, true);
+  return f > 0 && g > 0 ? b : 0;
+}
+
+int resident_clusters(int N) {
+#define NSGB_RESIDENT_CASE(NN, R, E)                                                  \
+  if (N == NN) {                                                                      \
+    const int n = probe_instances<NN, R, E, NSGB_SCHEME_CENTRAL>();                   \
+    const int m = probe_instances<NN, R, E, NSGB_SCHEME_UPWIND>();                    \
+    return n < m ? n : m;                                                             \
+  }
+  NSGB_RESIDENT(NSGB_RESIDENT_CASE)
+#undef NSGB_RESIDENT_CASE
+  return 0;
 }
 
 cudaError_t launch_resident(int N, const ResidentArgs& a, cudaStream_t st) {
-  return resident_dispatch(N, a, a.ckpt != nullptr, false, st);
+  const bool up = a.scheme == NSGB_SCHEME_UPWIND, grad = a.ckpt != nullptr;
+#define NSGB_RESIDENT_CASE(NN, R, E)                                                            \
+  if (N == NN) {                                                                                \
+    if (grad)                                                                                   \
+      return up ? launch_resident_t<NN, R, E, NSGB_SCHEME_UPWIND, true>(a, st)                  \
+                : launch_resident_t<NN, R, E, NSGB_SCHEME_CENTRAL, true>(a, st);                \
+    return up ? launch_resident_t<NN, R, E, NSGB_SCHEME_UPWIND, false>(a, st)                   \
+              : launch_resident_t<NN, R, E, NSGB_SCHEME_CENTRAL, false>(a, st);                 \
+  }
+  NSGB_RESIDENT(NSGB_RESIDENT_CASE)
+#undef NSGB_RESIDENT_CASE
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_resident_batch(int N, int scheme, const ResidentArgs* tab, int count, cudaStream_t st) {
+#define NSGB_RESIDENT_CASE(NN, R, E)                                                                     \
+  if (N == NN)                                                                                           \
+    return scheme == NSGB_SCHEME_UPWIND ? launch_resident_batch_t<NN, R, E, NSGB_SCHEME_UPWIND>(tab, count, st) \
+                                        : launch_resident_batch_t<NN, R, E, NSGB_SCHEME_CENTRAL>(tab, count, st);
+  NSGB_RESIDENT(NSGB_RESIDENT_CASE)
+#undef NSGB_RESIDENT_CASE
+  return cudaErrorInvalidValue;
 }
 
 NSGB_BOUNDS_UNIT(resident, 7)

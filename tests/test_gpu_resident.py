@@ -71,7 +71,7 @@ def test_gradients_equal_tiled_and_batched(nat, N, scheme, steps, every):
     J, g, uf, du = _grad(nat, u0, th, steps, every, sch)
     Jt, gt, uft, dut = _tiled(nat, N, lambda: _grad(nat, u0, th, steps, every, sch))
     assert torch.equal(uf, uft) and torch.equal(du, dut)
-    # one launch per kernel and tick, the same tiles: J and dJ/dtheta bit for bit
+    # in slices of five operations: J and dJ/dtheta bit for bit
     gb = GradientBatch()
     sid = gb.add(u0, th, steps, every, L, NU, DT, scheme, want_du0=True)
     gb.run(ops_per_call=5)
@@ -86,6 +86,48 @@ def test_single_steps_equal_the_tiled_step(nat, N):
         def step():
             return nat.op_step(u0, th, 0.37, L, NU, DT, sch, 0.5, 0.1, 1.0)
         assert torch.equal(step(), _tiled(nat, N, step))
+
+
+@pytest.mark.parametrize("N", SIZES)
+@pytest.mark.parametrize("ops", [1, 2, 3, 7])
+def test_sliced_gradients(nat, N, ops):
+    """Slices that end in every kind of operation take up the state of the one
+    before, members of unlike schedules, schemes and progress in one launch."""
+    from ns_solver_jax_differential_distributed_gb300.ensemble import GradientBatch
+    u0, th = _inputs(N)
+    want, gb, ids = [], GradientBatch(), []
+    for i, (steps, every) in enumerate([(7, 1), (7, 3), (8, 50), (9, 4), (1, 1)]):
+        want.append(_grad(nat, u0, th, steps, every, i % 2))
+        ids.append(gb.add(u0, th, steps, every, L, NU, DT, ["central", "upwind"][i % 2], want_du0=True,
+                          want_u_final=True))
+        gb.advance(ops)
+    gb.run(ops_per_call=ops)
+    for (J, g, uf, du), k in zip(want, ids):
+        Jb, gbt = gb.result(k)
+        assert torch.equal(J, Jb) and torch.equal(g, gbt)
+        assert torch.equal(uf, gb.u_final(k)) and torch.equal(du, gb.du0(k))
+
+
+def test_sliced_gradients_in_a_crowd(nat):
+    """Too many solves for their clusters run tick by tick: a solve that goes
+    from one way to the other and back keeps its bits."""
+    from ns_solver_jax_differential_distributed_gb300.ensemble import GradientBatch
+    u0, th = _inputs(128)
+    gb = GradientBatch()
+    first = gb.add(u0, th, 31, 5, L, NU, DT, "central", want_du0=True, want_u_final=True)
+    gb.advance(13)  # forward steps, alone
+    crowd = [gb.add(u0, th, 5, 5, L, NU, DT, "upwind") for _ in range(60)]
+    gb.advance(11)  # tick by tick; the crowd of 15 operations goes on
+    gb.advance(20)
+    gb.run(ops_per_call=9)
+    J, g, uf, du = _grad(nat, u0, th, 31, 5, 0)
+    Jb, gbt = gb.result(first)
+    assert torch.equal(J, Jb) and torch.equal(g, gbt)
+    assert torch.equal(uf, gb.u_final(first)) and torch.equal(du, gb.du0(first))
+    Jc, gc = _grad(nat, u0, th, 5, 5, 1)[:2]
+    for k in crowd:
+        Jb, gbt = gb.result(k)
+        assert torch.equal(Jc, Jb) and torch.equal(gc, gbt)
 
 
 def test_phases_one_by_one(nat):
