@@ -2142,7 +2142,14 @@ int nsgb_ensemble_rollout(const nsgb_member* members_in, int count, int chunk, v
   int s = 1;
   if (chunk > 0 && steps - 1 >= chunk) {
     std::lock_guard<std::mutex> lk(g_ens_mu);
-    const uint64_t sig = fnv(tab.data(), sizeof(SolveDev) * count);
+    // what the captured launches hold: the table's contents and the shapes
+    uint64_t sig = fnv(tab.data(), sizeof(SolveDev) * count);
+    for (const EnsGroup& G : groups) {
+      const nsgb_plan* p = G.plan;
+      const int shape[] = {p->N,           p->tile_w,       p->tile_h,    p->rows_per_cta,
+                           p->cols_per_cta, p->radix_rows, p->radix_cols, G.count};
+      sig = sig * 1099511628211ull ^ fnv(shape, sizeof shape);
+    }
     EnsGraph* eg = nullptr;
     for (auto& g : g_ens_graphs)
       if (g.ws == workspace && g.count == count && g.chunk == chunk && g.sig == sig) eg = &g;

@@ -51,3 +51,21 @@ def test_gradient_replays_with_other_buffers(nat, N, steps, every):
         assert torch.equal(J, Jb) and torch.equal(g, gr) and torch.equal(uf, gb.u_final(sid)), k
         assert du is None or torch.equal(du, gb.du0(sid)), k
         keep.append((u0, th, J, g, uf, du))
+
+
+def test_ensemble_graphs_follow_the_launch_shapes(nat):
+    """An ensemble run again on the same buffers after its plan's transforms
+    changed captures anew: the bits of solo solves of that plan."""
+    from ns_solver_jax_differential_distributed_gb300.ensemble import Ensemble, SolveSpec
+    plan, spec = nat.get_plan(64, L, torch.device("cuda")), spectral_u0(64, 8, 5)
+    ens = Ensemble([SolveSpec(N=64, u0=spec, theta=(0.9, 0.4), nu=NU, dt=DT, scheme="upwind")], steps=40)
+    u0, th = torch.from_numpy(spec).cuda(), torch.tensor([0.9, 0.4], device="cuda")
+    old = plan.fft_radix()
+    try:
+        for radix in ((8, 8), (16, 16), (8, 16)):
+            plan.set_fft_radix(*radix)
+            u = ens.run()[1][0]
+            us = nat.op_rollout(u0, th, 40, L, NU, DT, nat.SCHEME_IDS["upwind"], 0.5, 0.1, 1.0, True)[1]
+            assert torch.equal(u, us), radix
+    finally:
+        plan.set_fft_radix(*old)
