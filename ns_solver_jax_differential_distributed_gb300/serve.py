@@ -88,7 +88,11 @@ class Request:
 
     @property
     def latency(self):
-        return None if self.t_done is None else self.t_done - self.arrival
+        """Seconds from arrival -- or from admission, where a trace is not
+        served in real time and a request is admitted before its arrival."""
+        if self.t_done is None:
+            return None
+        return self.t_done - (self.arrival if self.t_admit is None else min(self.arrival, self.t_admit))
 
 
 # Time step of a request without an explicit one: the reference's stable step
