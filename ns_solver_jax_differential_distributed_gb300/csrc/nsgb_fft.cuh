@@ -286,10 +286,9 @@ __device__ __forceinline__ void pass(float2 (&a)[E], float2* __restrict__ sb, in
 
 // Full FFT of length N (unnormalised; INV uses exp(+2 pi i ...)) in radix E,
 // with `tw` the radix-E tables.  Every thread of the CTA (BAR = 0), or of the
-// N/E-thread warp group synchronised by barrier BAR, must call it: it
-// synchronises those threads between passes.  On return the exchange buffer
-// is free for reuse without a further barrier only after their next
-// synchronisation.
+// N/E-thread group synchronised by BAR, must call it: it synchronises those
+// threads between passes, the last time after their last read of the exchange
+// buffer, which is free for reuse on return.
 template <int N, bool INV, int E, int BAR = 0>
 __device__ __forceinline__ void block_fft(float2 (&a)[E], float2* sb, int j, const float2* __restrict__ tw) {
   pass<N, 1, INV, E, BAR>(a, sb, j, tw);

@@ -20,6 +20,17 @@ __host__ __device__ constexpr int pair_stride() {
   return padlen(N) + 2;
 }
 
+// How a pass kernel's transforms of T threads synchronise: within the warp
+// where they fit one (a step of 11 solves of N = 512 39.9 -> 39.3 us, of 30 of N
+// = 256 in radix 8 30.7 -> 30.1, against the CTA's barrier); else as a CTA:
+// hardware barriers of their own were slower (N = 512 in radix 8, 11 solves:
+// 44.5 against 41.9 us).  A persistent kernel (COH) has idle threads and always
+// meets as a CTA.
+template <int T, bool COH>
+__host__ __device__ constexpr int fft_bar() {
+  return T <= 32 && !COH ? -1 : 0;
+}
+
 // ---------------------------------------------------------------- rows fwd --
 // Transform thread j of row pair pp of a CTA carrying P row pairs, rows
 // [bx * 2P, +2P) (blockDim = (T, P): j = threadIdx.x, pp = threadIdx.y).  A
@@ -32,6 +43,7 @@ __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, flo
                                               const float2* __restrict__ tw, int j, int pp, int P, int bx) {
   constexpr int T = N / E;
   constexpr int H = N / 2;
+  constexpr int BAR = fft_bar<T, COH>();
   extern __shared__ float2 smem2[];
   float2* sb = smem2 + pp * pair_stride<N>();
   const int RB = 2 * P;
@@ -45,8 +57,7 @@ __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, flo
 #pragma unroll
   for (int s = 0; s < E; ++s)
     a[s] = make_float2(gldstream<COH>(ra + j + s * T), gldstream<COH>(rb + j + s * T));
-  fft::block_fft<N, false, E>(a, sb, j, tw);
-  __syncthreads();
+  fft::block_fft<N, false, E, BAR>(a, sb, j, tw);
   fft::store_strided<T, E>(a, sb, j);
   __syncthreads();
 
@@ -98,6 +109,7 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
                                           int bx) {
   constexpr int T = N / E;
   constexpr int H = N / 2;
+  constexpr int BAR = fft_bar<T, COH>();
   extern __shared__ float2 smem2[];
   float2* sb = smem2 + y * pair_stride<N>();
   // N/2 + 1 rows; the last CTA may hold rows past N/2, which recompute row
@@ -109,7 +121,7 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
   float2 a[E];
 #pragma unroll
   for (int s = 0; s < E; ++s) a[s] = gldstream<COH>(row + j + s * T);
-  fft::block_fft<N, false, E>(a, sb, j, tw);
+  fft::block_fft<N, false, E, BAR>(a, sb, j, tw);
 
   const float k2y = gldg(k2 + ky);
 #pragma unroll
@@ -119,7 +131,7 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
     // against 43.0 us at N = 4096)
     a[s] = make_float2(a[s].x * g, a[s].y * g);
   }
-  fft::block_fft<N, true, E>(a, sb, j, tw);
+  fft::block_fft<N, true, E, BAR>(a, sb, j, tw);
   __syncthreads();  // rows clamped to N/2 were loaded by other threads
   if (kreq <= H) {
 #pragma unroll
@@ -135,6 +147,7 @@ __device__ __forceinline__ void rows_inv_body(const float2* __restrict__ spec, f
                                               const float2* __restrict__ tw, int j, int pp, int P, int bx) {
   constexpr int T = N / E;
   constexpr int H = N / 2;
+  constexpr int BAR = fft_bar<T, COH>();
   extern __shared__ float2 smem2[];
   const int RB = 2 * P;
   const int i0 = bx * RB;
@@ -182,8 +195,8 @@ __device__ __forceinline__ void rows_inv_body(const float2* __restrict__ spec, f
   float2* sb = smem2 + pp * pair_stride<N>();
   float2 a[E];
   fft::load_strided<T, E>(a, sb, j);
-  __syncthreads();
-  fft::block_fft<N, true, E>(a, sb, j, tw);
+  fft::group_sync<BAR, T>();
+  fft::block_fft<N, true, E, BAR>(a, sb, j, tw);
   if (COH && pp >= P) return;
   float* ra = p + (size_t)(i0 + 2 * pp) * N;
   float* rb = ra + N;
