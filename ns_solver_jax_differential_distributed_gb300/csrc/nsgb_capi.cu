@@ -120,10 +120,13 @@ void default_tiles(int N, int sms, int out[4]) {
       if (out[1] >= 8) break;
     }
   }
-  int rows = N >= 1024 ? 4 : (N >= 256 ? 8 : 16);
+  // N = 2048: 8 rows a CTA against 4, 50.5 against 51.9 us a step; at 4096 183.6
+  // against 175.1.  One column a CTA from N = 512 on (two: 12.9 -> 13.0 us there,
+  // 4096 175 -> 185).
+  int rows = N == 1024 || N >= 4096 ? 4 : (N >= 256 ? 8 : 16);
   if (rows > N) rows = N;
   out[2] = rows;
-  int kb = N >= 1024 ? 1 : 4;
+  int kb = N >= 512 ? 1 : N >= 256 ? 2 : 4;
   if (kb > N / 2) kb = N / 2;
   out[3] = kb;
 }
@@ -969,7 +972,8 @@ int nsgb_plan_create(int N, double L, nsgb_plan** out) {
   }
   p->rows_per_cta = t[2];
   p->cols_per_cta = t[3];
-  p->radix_rows = p->radix_cols = fft_default_radix(N);
+  p->radix_rows = fft_default_radix_rows(N);
+  p->radix_cols = fft_default_radix_cols(N);
 
   // Per-pass twiddle tables of the Stockham FFT, radix 16 then radix 8
   // (layout in nsgb_fft.cuh).
