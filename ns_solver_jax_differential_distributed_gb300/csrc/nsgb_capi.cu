@@ -1198,6 +1198,10 @@ int nsgb_projector_step(const nsgb_plan* plan, const nsgb_phys* phys, const floa
   a.us = u;
   a.p = nullptr;
   a.f = f;
+  if ((uintptr_t)f & 15) {  // read as float4 groups
+    NSGB_CUDA(cudaMemcpyAsync(w.usB, f, 2 * sizeof(float) * plan->N * plan->N, cudaMemcpyDeviceToDevice, st));
+    a.f = w.usB;
+  }
   a.us_out = w.usA;
   a.rhs = w.rhs;
   a.t_from_step = 0;
@@ -1393,6 +1397,17 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
 }  // extern "C"
 
 namespace {
+// The last adjoint step stores float4 groups: into the caller's dJdu0 where that
+// is 16-byte aligned, else into its lambda buffer, from where it is copied.
+bool du0_direct(const float* dJdu0) { return dJdu0 && ((uintptr_t)dJdu0 & 15) == 0; }
+float* du0_target(float* dJdu0, const GradWs& g, int steps) {
+  return du0_direct(dJdu0) ? dJdu0 : (steps - 1) % 2 == 0 ? g.lamA : g.lamB;
+}
+cudaError_t du0_copy(float* dJdu0, const GradWs& g, int steps, size_t NN, cudaStream_t st) {
+  if (!dJdu0 || du0_direct(dJdu0)) return cudaSuccess;
+  return cudaMemcpyAsync(dJdu0, du0_target(dJdu0, g, steps), 2 * NN * sizeof(float), cudaMemcpyDeviceToDevice, st);
+}
+
 // One gradient call (validated arguments).  Its launches that touch the
 // caller's buffers -- the first forward step, the final state, the objective,
 // the last adjoint step and the sensitivities -- are enqueued one by one; what
@@ -1446,7 +1461,7 @@ struct GradCall {
     x.p = n == 0 ? nullptr : g.padj;
     // a one-step segment's state is its checkpoint
     x.u = s1 - s0 == 1 ? g.ckpt + (size_t)(s0 / every) * 2 * NN : g.ustore + (size_t)(s - s0) * 2 * NN;
-    x.lam_out = (s == 0 && dJdu0) ? dJdu0 : (n % 2 == 0 ? g.lamA : g.lamB);
+    x.lam_out = s == 0 ? du0_target(dJdu0, g, steps) : (n % 2 == 0 ? g.lamA : g.lamB);
     x.step = s;
     return x;
   }
@@ -1568,10 +1583,13 @@ int nsgb_rollout_grad(const nsgb_plan* plan, const nsgb_phys* phys, const float*
                                         (phases & NSGB_GRAD_BACKWARD) ? grad_ops_total(steps, every) : steps);
     r.u0 = u0;
     r.u_final = u_final;
-    r.dJdu0 = dJdu0;
+    if (dJdu0) r.dJdu0 = du0_target(dJdu0, g, steps);
     NSGB_CUDA(launch_resident(plan->N, r, st));
     if (phases & NSGB_GRAD_FORWARD) NSGB_CUDA(launch_jreduce(g.f.jpart, nblk, steps, g.f.jsteps, J, jscale, st));
-    if (phases & NSGB_GRAD_BACKWARD) NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
+    if (phases & NSGB_GRAD_BACKWARD) {
+      NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
+      NSGB_CUDA(du0_copy(dJdu0, g, steps, call.NN, st));
+    }
     return finish_call(st);
   }
 
@@ -1586,6 +1604,7 @@ int nsgb_rollout_grad(const nsgb_plan* plan, const nsgb_phys* phys, const float*
     if (int r = grad_part(pl, call, 1, workspace, st)) return r;
     NSGB_CUDA(launch_adjoint_stencil(call.adjoint_args(0, 0, std::min(steps, every), dJdu0), st));
     NSGB_CUDA(launch_gsum(g.gpart, adj_nblk, theta_len, dJdtheta, st));
+    NSGB_CUDA(du0_copy(dJdu0, g, steps, call.NN, st));
   }
   return finish_call(st);
 }
@@ -1744,7 +1763,7 @@ AdjointArgs grad_adj_args(const nsgb_grad_member& m, const GradMemberCtx& c, con
   x.lam = b == 0 ? nullptr : (((b - 1) % 2 == 0) ? c.g.lamA : c.g.lamB);
   x.p = b >= 1 ? c.g.padj : nullptr;
   x.u = (o.s1 - o.s0 == 1) ? c.g.ckpt + (size_t)o.seg * 2 * c.NN : c.g.ustore + (size_t)(s - o.s0) * 2 * c.NN;
-  x.lam_out = (s == 0 && m.dJdu0) ? m.dJdu0 : ((b % 2 == 0) ? c.g.lamA : c.g.lamB);
+  x.lam_out = s == 0 ? du0_target(m.dJdu0, c.g, m.steps) : ((b % 2 == 0) ? c.g.lamA : c.g.lamB);
   x.step = s;
   return x;
 }
@@ -1824,7 +1843,7 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
         ResidentArgs r = resident_grad_args(plan, ctx[i].a, ctx[i].g, m.steps, m.every, op0, op1);
         r.u0 = m.u0;
         r.u_final = m.u_final;
-        r.dJdu0 = m.dJdu0;
+        if (m.dJdu0) r.dJdu0 = du0_target(m.dJdu0, ctx[i].g, m.steps);
         tab[m.phys.scheme == NSGB_SCHEME_CENTRAL ? 0 : 1].push_back(r);
         GradAction z{};
         z.group = gi;
@@ -1966,6 +1985,7 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
         const nsgb_grad_member& m = members[z.member];
         const GradMemberCtx& c = ctx[z.member];
         NSGB_CUDA(launch_gsum(c.g.gpart, c.adj_nblk, m.theta_len, m.dJdtheta, st));
+        NSGB_CUDA(du0_copy(m.dJdu0, c.g, m.steps, c.NN, st));
         break;
       }
     }
