@@ -26,6 +26,7 @@
 // over a thread's few cells and in double from there on.
 #include "nsgb_adjoint_cell.cuh"
 #include "nsgb_rows.cuh"
+#include "nsgb_stencil_body.cuh"
 
 namespace nsgb {
 
@@ -205,14 +206,194 @@ __device__ __forceinline__ void adjoint_body(const AdjointArgs& a) {
   }
 }
 
+// Tiles at least 64 wide: four cells per thread, as the wide forward tiles
+// (nsgb_stencil_body.cuh), asynchronous loads, 16-byte shared-memory accesses
+// and stores: shared-memory instructions bound the one-cell body.  A forward and
+// an adjoint step at the default tile, N = 256 20.0 -> 19.5 us, 512 27.6 -> 26.5;
+// at 1024 in 128 x 8 tiles 50.1 -> 47.5 (its default are the row bands below).
+template <int TW, int TH>
+struct Adjoint4Smem {
+  static constexpr int G = TW / 4 + 2;        // groups per row
+  static constexpr int W4 = 4 * G;
+  static constexpr int PH = TH + 6, UH = TH + 4, SH = TH + 2;
+  static constexpr int NT = tile_threads<TW, TH>();
+  static constexpr int P_OFF = 4;                     // PH rows (4 floats before: the first row's left neighbour)
+  static constexpr int UX_OFF = P_OFF + PH * W4;      // UH rows each
+  static constexpr int UY_OFF = UX_OFF + UH * W4;
+  static constexpr int MX_OFF = UY_OFF + UH * W4;
+  static constexpr int MY_OFF = MX_OFF + UH * W4;
+  static constexpr int LX_OFF = MY_OFF + UH * W4;     // SH rows each
+  static constexpr int LY_OFF = LX_OFF + SH * W4;
+  static constexpr int F_OFF = LY_OFF + SH * W4 + 4;  // fx of the SH rows
+  static constexpr int DA_OFF = F_OFF + SH;           // dfx/dA, dfx/dB of the TH rows
+  static constexpr int DB_OFF = DA_OFF + TH;
+  static constexpr int RED_OFF = (DB_OFF + TH + 1) & ~1;  // 3 x 8 double-floats
+  static constexpr size_t BYTES = (size_t)RED_OFF * sizeof(float) + 24 * sizeof(DFloat);
+  static_assert(NT % 32 == 0 && NT <= 256 && NT >= 64 + TH && SH <= 64, "threads");
+};
+
 template <int SCHEME, int TW, int TH>
-__global__ void __launch_bounds__(256) k_adjoint(const AdjointArgs a) {
-  adjoint_body<SCHEME, TW, TH>(a);
+__device__ __forceinline__ void adjoint4_body(const AdjointArgs& a) {
+  using Lay = Adjoint4Smem<TW, TH>;
+  constexpr int G = Lay::G, W4 = Lay::W4, PH = Lay::PH, UH = Lay::UH, SH = Lay::SH, NT = Lay::NT;
+  extern __shared__ __align__(16) float sm[];
+  float* sP = sm + Lay::P_OFF;
+  float* sUx = sm + Lay::UX_OFF;
+  float* sUy = sm + Lay::UY_OFF;
+  float* sMx = sm + Lay::MX_OFF;
+  float* sMy = sm + Lay::MY_OFF;
+  float* sLx = sm + Lay::LX_OFF;
+  float* sLy = sm + Lay::LY_OFF;
+  float* sF = sm + Lay::F_OFF;
+  float* sDA = sm + Lay::DA_OFF;
+  float* sDB = sm + Lay::DB_OFF;
+  DFloat* sRed = reinterpret_cast<DFloat*>(sm + Lay::RED_OFF);
+  const StepConsts& c = a.c;
+  const int N = c.N, M = N - 1;
+  const size_t NN = (size_t)N * N;
+  const int j0 = blockIdx.x * TW, i0 = blockIdx.y * TH;
+  const int tid = threadIdx.x;
+  const bool has_lam = a.lam != nullptr;
+  const bool has_p = a.p != nullptr;
+
+#pragma unroll
+  for (int e = tid; e < UH * G; e += NT) {
+    const int r = e / G, q = e % G;
+    const size_t g = (size_t)((i0 - 2 + r) & M) * N + ((j0 - 4 + 4 * q) & M);
+    copy16(sUx + 4 * e, a.u + g);
+    copy16(sUy + 4 * e, a.u + NN + g);
+    if (has_lam) {
+      copy16(sMx + 4 * e, a.lam + g);
+      copy16(sMy + 4 * e, a.lam + NN + g);
+    } else {
+      *reinterpret_cast<float4*>(sMx + 4 * e) = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(sMy + 4 * e) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  if (has_p) {
+#pragma unroll
+    for (int e = tid; e < PH * G; e += NT) {
+      const int r = e / G, q = e % G;
+      copy16(sP + 4 * e, a.p + (size_t)((i0 - 3 + r) & M) * N + ((j0 - 4 + 4 * q) & M));
+    }
+  }
+  const float dt = c.dt;
+  const float jscale = c.jscale;  // float32(dt * dx^2) = dJ/du_x / f_x
+  {
+    const float t = fmul((float)a.step, dt);
+    const float A = gldg(a.theta), B = gldg(a.theta + 1);
+    const ForcingRow fr = forcing_time(A, B, t, c);
+    if (tid < SH)
+      sF[tid] = forcing_fx((i0 - 1 + tid) & M, fr, c);
+    else if (tid >= 64 && tid < 64 + TH)
+      forcing_theta_grad((i0 + tid - 64) & M, fr, A, B, t, c, sDA[tid - 64], sDB[tid - 64]);
+  }
+  const float nu = (a.theta_len == 3) ? gldg(a.theta + 2) : c.nu;
+  const float cL = fmul(c.dtdx2, nu);                              // dt nu / dx^2
+  const float cA = SCHEME == NSGB_SCHEME_CENTRAL ? c.cAc : c.cAu;  // dt / h
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+
+  // mu = lambda - dt grad p on rows i0-2 .. i0+TH+1
+  if (has_p) {
+    project4<UH, G, NT>(sMx, sMy, sP, c.cP, tid);
+    __syncthreads();
+  }
+
+  // lambda_s on rows i0-1 .. i0+TH
+#pragma unroll 1
+  for (int e = tid; e < SH * G; e += NT) {
+    struct Cells {
+      float s[4], o[6], n[4];
+      __device__ __forceinline__ AdjNbr at(int k) const { return {o[k + 1], n[k], s[k], o[k + 2], o[k]}; }
+    } mx, my, ux, uy;
+    auto cells = [&](const float* f, Cells& d) {  // row e / G of f: one row up
+      get4(f + 4 * e, d.s);
+      get6(f + 4 * e + W4, d.o);
+      get4(f + 4 * e + 2 * W4, d.n);
+    };
+    cells(sMx, mx);
+    cells(sMy, my);
+    cells(sUx, ux);
+    cells(sUy, uy);
+    const float fterm = jscale * sF[e / G];
+    float lx[4], ly[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      adjoint_cell<SCHEME>(mx.at(k), my.at(k), ux.at(k), uy.at(k), cL, cA, fterm, lx[k], ly[k]);
+    set4(sLx + 4 * e, lx);
+    set4(sLy + 4 * e, ly);
+  }
+
+  // theta sensitivities of the thread's own cells (adjoint_body): float over
+  // two cells, double-float across the block
+  const int r = tid / (TW / 4), q = tid % (TW / 4) + 1;
+  DFloat vA, vB, vN;
+  {
+    const int o = (r + 2) * W4 + 4 * q;
+    float mx[4], my[4], ux[6], uy[6], us[4], un[4], vs[4], vn[4];
+    get4(sMx + o, mx);
+    get4(sMy + o, my);
+    get6(sUx + o, ux);
+    get4(sUx + o - W4, us);
+    get4(sUx + o + W4, un);
+    get6(sUy + o, uy);
+    get4(sUy + o - W4, vs);
+    get4(sUy + o + W4, vn);
+    float fA[2] = {0.f, 0.f}, fB[2] = {0.f, 0.f}, fN[2] = {0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int h = k / 2;
+      const float ox = ux[k + 1], oy = uy[k + 1];
+      const float w = fmaf(jscale, ox, dt * mx[k]);
+      fA[h] = fmaf(w, sDA[r], fA[h]);
+      fB[h] = fmaf(w, sDB[r], fB[h]);
+      const float lux = ((us[k] - ox) + (un[k] - ox)) + ((ux[k + 2] - ox) + (ux[k] - ox));
+      const float luy = ((vs[k] - oy) + (vn[k] - oy)) + ((uy[k + 2] - oy) + (uy[k] - oy));
+      fN[h] = fmaf(mx[k], lux, fmaf(my[k], luy, fN[h]));
+    }
+    vA = df_add({fA[0], 0.f}, {fA[1], 0.f});
+    vB = df_add({fB[0], 0.f}, {fB[1], 0.f});
+    vN = df_add({fN[0], 0.f}, {fN[1], 0.f});
+  }
+  const int lane = tid & 31;
+  // lanes 0-7: A, 16-23: B, 8-15 and 24-31: nu
+  DFloat v = fold<8>(fold<16>(vA, vB, lane), fold1(vN, 16), lane);
+  v = fold1(fold1(fold1(v, 4), 2), 1);
+  if (lane % 8 == 0 && lane < 24) sRed[(lane == 0 ? 0 : lane == 16 ? 8 : 16) + tid / 32] = v;
+  __syncthreads();
+
+  const size_t g = (size_t)(i0 + r) * N + (j0 - 4 + 4 * q);
+  const int os = (r + 1) * W4 + 4 * q;
+  float x[4], y[4];
+  get4(sLx + os, x);
+  get4(sLy + os, y);
+  gst4(a.lam_out + g, make_float4(x[0], x[1], x[2], x[3]));
+  gst4(a.lam_out + NN + g, make_float4(y[0], y[1], y[2], y[3]));
+  gst4(a.rhs + g, rhs4<W4>(sLx + os, sLy + os, c.cD));
+  if (tid < 32) {
+    DFloat s = tid < 24 && tid % 8 < NT / 32 ? sRed[tid] : DFloat{0.f, 0.f};
+    s = fold1(fold1(fold1(s, 4), 2), 1);  // lanes 0, 8, 16: A, B, nu
+    const DFloat s1 = {__shfl_sync(0xffffffffu, s.hi, 8), __shfl_sync(0xffffffffu, s.lo, 8)};
+    const DFloat s2 = {__shfl_sync(0xffffffffu, s.hi, 16), __shfl_sync(0xffffffffu, s.lo, 16)};
+    if (tid == 0) add_theta_partials(a, blockIdx.y * gridDim.x + blockIdx.x, s, s1, s2);
+  }
+}
+
+template <int SCHEME, int TW, int TH>
+__global__ void __launch_bounds__((tile_threads<TW, TH>())) k_adjoint(const AdjointArgs a) {
+  if constexpr (wide_tile<TW>())
+    adjoint4_body<SCHEME, TW, TH>(a);
+  else
+    adjoint_body<SCHEME, TW, TH>(a);
 }
 // Batched form: blockIdx.z selects the solve's arguments.
 template <int SCHEME, int TW, int TH>
-__global__ void __launch_bounds__(256) k_adjoint_b(const AdjointArgs* __restrict__ tab) {
-  adjoint_body<SCHEME, TW, TH>(tab[blockIdx.z]);
+__global__ void __launch_bounds__((tile_threads<TW, TH>())) k_adjoint_b(const AdjointArgs* __restrict__ tab) {
+  if constexpr (wide_tile<TW>())
+    adjoint4_body<SCHEME, TW, TH>(tab[blockIdx.z]);
+  else
+    adjoint_body<SCHEME, TW, TH>(tab[blockIdx.z]);
 }
 
 // a: the shape, scheme and N of the launch; tab (device, count entries) or
@@ -222,10 +403,12 @@ static cudaError_t launch_adjoint_t(const AdjointArgs& a, const AdjointArgs* tab
   const cudaError_t e = tab ? raise_smem_limit(k_adjoint_b<SCHEME, TW, TH>) : raise_smem_limit(k_adjoint<SCHEME, TW, TH>);
   if (e != cudaSuccess) return e;
   const dim3 grid(a.c.N / TW, a.c.N / TH, tab ? count : 1);
+  const dim3 block = wide_tile<TW>() ? dim3(tile_threads<TW, TH>()) : dim3(32, 8);
+  const size_t smem = wide_tile<TW>() ? Adjoint4Smem<TW, TH>::BYTES : AdjointSmem<TW, TH>::BYTES;
   if (tab)
-    k_adjoint_b<SCHEME, TW, TH><<<grid, dim3(32, 8), AdjointSmem<TW, TH>::BYTES, st>>>(tab);
+    k_adjoint_b<SCHEME, TW, TH><<<grid, block, smem, st>>>(tab);
   else
-    k_adjoint<SCHEME, TW, TH><<<grid, dim3(32, 8), AdjointSmem<TW, TH>::BYTES, st>>>(a);
+    k_adjoint<SCHEME, TW, TH><<<grid, block, smem, st>>>(a);
   return cudaGetLastError();
 }
 

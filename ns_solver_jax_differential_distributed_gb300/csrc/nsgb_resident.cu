@@ -107,19 +107,6 @@ __device__ __forceinline__ void st_remote4(uint32_t a, float x, float y, float z
                : "memory");
 }
 
-// Half of a warp-wide double-float sum serves two values: lanes with bit O
-// clear go on with x's partials, the others with y's.  df_add does not depend
-// on its operands' order, so each value's tree is that of warp_sum_df.
-template <int O>
-__device__ __forceinline__ DFloat fold(DFloat x, DFloat y, int lane) {
-  const bool up = (lane & O) != 0;
-  const DFloat keep = up ? y : x, give = up ? x : y;
-  return df_add(keep, {__shfl_xor_sync(0xffffffffu, give.hi, O), __shfl_xor_sync(0xffffffffu, give.lo, O)});
-}
-__device__ __forceinline__ DFloat fold1(DFloat v, int o) {
-  return df_add(v, {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
-}
-
 template <int N, int R, int E, int SCHEME, bool GRAD>
 struct Solve {
   using L = Lay<N, R, E>;

@@ -22,17 +22,6 @@
 
 namespace nsgb {
 
-// Tiles at least 64 wide use the body with four cells per thread (a block of
-// TW/4 x TH threads in one dimension), narrower ones a block of 32 x 8.
-template <int TW>
-constexpr bool wide_tile() {
-  return TW >= 64;
-}
-template <int TW, int TH>
-constexpr int tile_threads() {
-  return wide_tile<TW>() ? TW / 4 * TH : 256;
-}
-
 template <int SCHEME, int MODE, int TW, int TH>
 __global__ void __launch_bounds__((tile_threads<TW, TH>())) k_stencil(const StencilArgs a) {
   if constexpr (wide_tile<TW>())

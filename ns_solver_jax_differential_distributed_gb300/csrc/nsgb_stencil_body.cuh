@@ -199,6 +199,17 @@ struct Stencil4Smem {
   static_assert(NT % 32 == 0 && NT <= 256, "threads");
 };
 
+// Tiles at least 64 wide use the body with four cells per thread (a block of
+// TW/4 x TH threads in one dimension), narrower ones a block of 32 x 8.
+template <int TW>
+constexpr bool wide_tile() {
+  return TW >= 64;
+}
+template <int TW, int TH>
+constexpr int tile_threads() {
+  return wide_tile<TW>() ? TW / 4 * TH : 256;
+}
+
 // Asynchronous 16-byte copy into shared memory through L2.
 __device__ __forceinline__ void copy16(float* dst, const float* src, int line = __builtin_LINE()) {
   if (!bounds_ok(src, 16, line)) return;

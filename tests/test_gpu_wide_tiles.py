@@ -38,3 +38,32 @@ def test_wide_tiles_equal_narrow_ones(cuda_lib, N, tile, scheme):
         plan.set_adjoint_tiles(*old_adj)
     assert torch.equal(uw, un) and torch.equal(pw, pn)
     assert abs(Jw - Jn) <= 1e-5 * abs(Jn) + 1e-9, (Jw, Jn)
+
+
+@pytest.mark.parametrize("scheme", [0, 1])
+@pytest.mark.parametrize("N,tile", [(64, (64, 8)), (64, (64, 16)), (128, (128, 8)), (256, (64, 16)), (256, (128, 8)),
+                                    (512, (64, 8))])
+def test_wide_adjoint_tiles_equal_narrow_ones(cuda_lib, N, tile, scheme):
+    """dJ/du0 bit for bit; dJ/dA and dJ/dB to the rounding of float sums of at
+    most eight cells (16 x 8 tiles have one cell per thread), 8 x 2^-24 of the
+    summed magnitudes, taken as at most 20 times the larger of the two (dJ/dnu is
+    a small difference of large terms, which no such bound holds)."""
+    from ns_solver_jax_differential_distributed_gb300 import _native as nat
+    dev = torch.device("cuda")
+    u0 = torch.from_numpy(spectral_u0(N, 8, N)).cuda()
+    th = torch.tensor([0.9, 0.4, 2e-3], device="cuda")
+    plan = nat.get_plan(N, L, dev)
+    old, old_adj = plan.tiles(), plan.adjoint_tiles()
+
+    def run(w, h):
+        plan.set_tiles(16, 8, old[2], old[3])
+        plan.set_adjoint_tiles(w, h)
+        return nat.rollout_grad_raw(u0, th, 6, 4, L, NU, DT, scheme, want_du0=True, own_workspace=True)
+    try:
+        _, gw, _, dw = run(*tile)
+        _, gn, _, dn = run(16, 8)
+    finally:
+        plan.set_tiles(*old)
+        plan.set_adjoint_tiles(*old_adj)
+    assert torch.equal(dw, dn)
+    assert (gw - gn)[:2].abs().max().item() <= 20 * 8 * 2.0 ** -24 * gn.abs().max().item(), (gw, gn)
