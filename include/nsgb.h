@@ -190,10 +190,12 @@ int nsgb_rollout(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0, 
  * call must follow a forward call with the same arguments and workspace
  * (the checkpoints live in the workspace).  The forward phase writes *J and,
  * if non-NULL, u_final; the backward phase writes dJdtheta[theta_len] and, if
- * non-NULL, dJdu0 (2,N,N).  A call repeated with the same arguments (pointers,
- * sizes, physics, launch shapes) is captured as one CUDA graph on its second
- * use and replayed after that, with the same results; inside a caller's own
- * stream capture the work is recorded eagerly.  Workspace:
+ * non-NULL, dJdu0 (2,N,N).  Small grids (32 to 128, default launch shapes) run
+ * as one launch.  Elsewhere a call repeated with the same workspace, sizes,
+ * physics and launch shapes has its inner steps captured as CUDA graphs on its
+ * second use and replayed after that, for any u0, theta and outputs, with the
+ * same results; inside a caller's own stream capture the work is recorded
+ * eagerly.  Workspace:
  * nsgb_rollout_grad_workspace_bytes(plan, steps, every) (it depends on the
  * plan's adjoint shape). */
 int nsgb_rollout_grad(const nsgb_plan* plan, const nsgb_phys* phys, const float* u0,
@@ -300,8 +302,9 @@ int nsgb_ensemble_advance(const nsgb_member* members, int count, int steps, void
 /* One-shot ensemble: all members start from u0 (done_steps ignored) and run
  * total_steps (equal for all members).  Chunks of `chunk` steps (even; 0 =
  * direct launches) are replayed as ONE CUDA graph per chunk in which the
- * groups run as parallel branches; `workspace` must stay the same between
- * calls for the cached graph to be reused. */
+ * groups run as parallel branches; `workspace`, the members and the plans'
+ * launch shapes must stay the same between calls for the cached graph to be
+ * reused. */
 int nsgb_ensemble_rollout(const nsgb_member* members, int count, int chunk, void* workspace,
                           size_t workspace_bytes, void* stream);
 

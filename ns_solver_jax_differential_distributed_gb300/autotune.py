@@ -10,6 +10,10 @@ cold L2 for grids larger than L2) and keeps the fastest per stage:
   inverse),
 * Stockham radix and spectrum rows per CTA of the column FFT.
 
+A plan that is not tuned starts from the library's measured defaults.  At the
+sizes of the resident kernel (N = 32 to 128), which runs at one shape only,
+the winner must also beat the default shape over a whole rollout.
+
 Results are cached in a JSON file keyed by GPU name, N and scheme
 (``$NSGB_TUNE_CACHE`` or ``<package>/_autotune/tiles.json``) so a process
 tunes a size once.  The stages are independent kernels, so each shape is
