@@ -104,8 +104,8 @@ namespace {
 //
 // Stencil: tiles up to N = 512, where a grid has too few rows for bands that
 // fill the GPU (N = 512: 8.4 us tiled, 9.4 us in bands); row bands from N = 1024
-// on (in the step, central, tiles of 64 x 16 against bands: N = 1024 14.4 ->
-// 12.4 us, 2048 39 -> 26.6, 4096 133 -> 70.1).  Bands of 1024 columns, two CTAs
+// on (a step, central, tiles of 64 x 16 against bands: N = 1024 21.0 -> 20.0 us,
+// 2048 55.3 -> 51.1).  Bands of 1024 columns, two CTAs
 // per SM in one wave, while they are at least 8 rows tall (each recomputes four
 // rows of its neighbours; at N = 1024 one CTA per SM, 7 rows, beats two of 4
 // rows: 12.4 against 13.7 us); at N = 8192 bands of 2048 columns, one CTA per SM
