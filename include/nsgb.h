@@ -88,8 +88,8 @@ int nsgb_plan_get_tiles(const nsgb_plan* plan, int out[4]);
 
 /* No counterpart in the reference (launch tuning).  Stockham radix (16 or 8)
  * of the row passes and of the column pass of the FFT-Poisson solve; 0 keeps
- * the current value.  Radix 8 carries a transform on twice as many threads
- * with half the registers each.  Results agree to FFT rounding. */
+ * the current value; plans start with radix 16.  Results agree to FFT
+ * rounding. */
 int nsgb_plan_set_fft_radix(nsgb_plan* plan, int radix_rows, int radix_cols);
 int nsgb_plan_get_fft_radix(const nsgb_plan* plan, int out[2]);
 

@@ -682,11 +682,10 @@ int plan_clusters(const nsgb_plan* plan) {
 }
 
 // Whether a plan's rollouts (grad: and gradients) run as resident launches: N
-// has an instance, the launch shapes are those it reproduces (32 x 8 tiles, its
-// radix), and the device can place its clusters.
+// has an instance, the launch shapes are those it reproduces (32 x 8 tiles,
+// radix 16), and the device can place its clusters.
 bool resident_plan(const nsgb_plan* plan, bool grad) {
-  const int radix = resident_radix(plan->N);
-  if (!radix || plan->radix_rows != radix || plan->radix_cols != radix) return false;
+  if (!resident_size(plan->N) || plan->radix_rows != 16 || plan->radix_cols != 16) return false;
   if (plan->tile_w != 32 || plan->tile_h != 8) return false;
   if (grad && (plan->adj_w != 32 || plan->adj_h != 8)) return false;
   return plan_clusters(plan) > 0;
@@ -697,7 +696,7 @@ ResidentArgs resident_args(const nsgb_plan* plan, const StencilArgs& a, const Ro
   ResidentArgs r;
   r.c = a.c;
   r.scheme = a.scheme;
-  r.tw = plan->tw + (resident_radix(plan->N) == 8 ? nsgb::fft::tw8_offset(plan->N) : 0);
+  r.tw = plan->tw;  // radix-16 tables first
   r.k2 = plan->k2;
   r.scale = plan->scale;
   r.theta = a.theta;
@@ -972,8 +971,6 @@ int nsgb_plan_create(int N, double L, nsgb_plan** out) {
   }
   p->rows_per_cta = t[2];
   p->cols_per_cta = t[3];
-  p->radix_rows = fft_default_radix_rows(N);
-  p->radix_cols = fft_default_radix_cols(N);
 
   // Per-pass twiddle tables of the Stockham FFT, radix 16 then radix 8
   // (layout in nsgb_fft.cuh).

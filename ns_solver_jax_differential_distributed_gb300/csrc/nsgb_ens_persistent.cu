@@ -70,15 +70,15 @@ __device__ bool grid_barrier(unsigned* bar, unsigned limit) {
 
 template <int N>
 __device__ __forceinline__ void rows_fwd_item(const FftPtrs& f, const PersMember& pm, int tid, int u) {
-  rows_fwd_body<N, 16, true>(f.rhs, f.spec, pm.tw, tid % fft_T(N), tid / fft_T(N), rows_P(N), u);
+  rows_fwd_body<N, 16, 16, true>(f.rhs, f.spec, pm.tw, tid % fft_T(N), tid / fft_T(N), rows_P(N), u);
 }
 template <int N>
 __device__ __forceinline__ void cols_item(const FftPtrs& f, const PersMember& pm, int tid, int u) {
-  cols_body<N, 16, true>(f.spec, pm.tw, pm.k2, pm.scale, tid % fft_T(N), tid / fft_T(N), cols_KB(N), u);
+  cols_body<N, 16, 16, true>(f.spec, pm.tw, pm.k2, pm.scale, tid % fft_T(N), tid / fft_T(N), cols_KB(N), u);
 }
 template <int N>
 __device__ __forceinline__ void rows_inv_item(const FftPtrs& f, const PersMember& pm, int tid, int u) {
-  rows_inv_body<N, 16, true>(f.spec, f.p, pm.tw, tid % fft_T(N), tid / fft_T(N), rows_P(N), u);
+  rows_inv_body<N, 16, 16, true>(f.spec, f.p, pm.tw, tid % fft_T(N), tid / fft_T(N), rows_P(N), u);
 }
 
 #define NSGB_PERS_SIZES(X) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)

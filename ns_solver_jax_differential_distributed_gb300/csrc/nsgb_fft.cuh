@@ -1,7 +1,8 @@
 // Block-level FFT building blocks for power-of-two lengths 16..4096.
 //
 // A transform of length N is carried by T = N/E threads, each holding E
-// complex values in registers (E = 16 or 8, at most N).  Thread j holds elements j + s*T
+// complex values in registers (E = 16 or 8, at most N; E the radix, or half a
+// radix of 16).  Thread j holds elements j + s*T
 // (s = 0..E-1) on entry and X[j + s*T] on exit, so the first pass reads and
 // the last pass writes "natural" strided positions; rows stored contiguously
 // in global memory are therefore loaded and stored fully coalesced.
@@ -77,11 +78,12 @@ __device__ __forceinline__ float2 rot16(float2 d, int m) {
   return make_float2(d.x * c - d.y * s, d.x * s + d.y * c);
 }
 
-// In-register DFT of size R (2, 4, 8 or 16): natural order in and out.
-template <int R, bool INV>
+// Stages of span LEN, LEN/2, .. 2 of the in-register DFT of size R (2, 4, 8 or
+// 16; LEN = R: the whole DFT), natural order in and out.
+template <int R, bool INV, int LEN = R>
 __device__ __forceinline__ void dft(float2 (&a)[R]) {
 #pragma unroll
-  for (int len = R; len >= 2; len >>= 1) {
+  for (int len = LEN; len >= 2; len >>= 1) {
     const int half = len >> 1;
 #pragma unroll
     for (int s = 0; s < R; s += len) {
@@ -99,6 +101,26 @@ __device__ __forceinline__ void dft(float2 (&a)[R]) {
   for (int k = 0; k < R; ++k) b[k] = a[bitrev<R>(k)];
 #pragma unroll
   for (int k = 0; k < R; ++k) a[k] = b[k];
+}
+
+// Sum and difference of u g and v h: the first butterfly of a transform whose
+// inputs are multiplied by a spectral multiplier.  The products are rounded,
+// but for the second one of a transform's last pair (last), which is fused.
+// Spelled out, because the fusing a compiler finds for itself changes from
+// kernel to kernel and with it the last bits of a solve, and an upwind gradient
+// is not continuous in those: a cell of |u| below them takes the other
+// one-sided difference in the adjoint step.
+__device__ __forceinline__ void scaled_butterfly(float2 u, float g, float2 v, float h, bool last, float2& sum,
+                                                 float2& dif) {
+  const float ux = fmul(u.x, g), uy = fmul(u.y, g);
+  if (last) {
+    sum = make_float2(__fmaf_rn(v.x, h, ux), __fmaf_rn(v.y, h, uy));
+    dif = make_float2(__fmaf_rn(-v.x, h, ux), __fmaf_rn(-v.y, h, uy));
+  } else {
+    const float vx = fmul(v.x, h), vy = fmul(v.y, h);
+    sum = make_float2(fadd(ux, vx), fadd(uy, vy));
+    dif = make_float2(fsub(ux, vx), fsub(uy, vy));
+  }
 }
 
 // Offset (in complex entries) of the twiddle table of the pass with stride
@@ -203,76 +225,202 @@ __device__ __forceinline__ void group_sync() {
   }
 }
 
-// One Stockham pass (stride NS) and, recursively, the remaining passes.
-template <int N, int NS, bool INV, int E, int BAR = 0>
-__device__ __forceinline__ void pass(float2 (&a)[E], float2* __restrict__ sb, int j,
+// a b, each part one rounded product and one fused; the imaginary part fuses
+// a.x b.y or (cmul_y) a.y b.x.
+__device__ __forceinline__ float2 cmul_x(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -fmul(a.y, b.y)), __fmaf_rn(a.x, b.y, fmul(a.y, b.x)));
+}
+__device__ __forceinline__ float2 cmul_y(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -fmul(a.y, b.y)), __fmaf_rn(a.y, b.x, fmul(a.x, b.y)));
+}
+// Products with a twiddle of the table, and of two of them.
+template <bool INV>
+__device__ __forceinline__ float2 cmul_tw(float2 a, float2 w) {
+  return INV ? cmul_y(a, w) : cmul_x(a, w);
+}
+
+// W^1, W^2, W^4, W^8 of position bm of a radix-16 pass (conjugate if INV).
+// W^r is one of them or the product of at most three (a few ulps), so a
+// radix-16 pass issues 4 twiddle loads instead of 15.
+template <int NS, bool INV>
+__device__ __forceinline__ void load_twiddles16(const float2* __restrict__ tw, int bm, float2& w1, float2& w2,
+                                                float2& w4, float2& w8) {
+  const float2* __restrict__ tp = tw + tw_offset<16>(NS) + bm;
+  w1 = gldg(tp + NS), w2 = gldg(tp + 2 * NS), w4 = gldg(tp + 4 * NS), w8 = gldg(tp + 8 * NS);
+  if (INV) {
+    w1.y = -w1.y;
+    w2.y = -w2.y;
+    w4.y = -w4.y;
+    w8.y = -w8.y;
+  }
+}
+
+// Twiddled inputs x[r] *= W^r of a butterfly of size RP at position bm of the
+// pass with stride NS, from the radix-R tables.  The radix-16 products are
+// spelled out, as in scaled_butterfly: half_butterfly forms the same ones.
+template <int NS, int RP, int R, bool INV>
+__device__ __forceinline__ void twiddle(float2 (&x)[RP], int bm, const float2* __restrict__ tw) {
+  if constexpr (RP == 16) {
+    float2 w1, w2, w4, w8;
+    load_twiddles16<NS, INV>(tw, bm, w1, w2, w4, w8);
+    const float2 w3 = cmul_tw<INV>(w2, w1), w12 = cmul_tw<INV>(w8, w4);
+    x[1] = cmul_tw<INV>(x[1], w1);
+    x[2] = cmul_tw<INV>(x[2], w2);
+    x[3] = cmul_x(x[3], w3);
+    x[4] = cmul_tw<INV>(x[4], w4);
+    x[5] = cmul_x(x[5], cmul_tw<INV>(w4, w1));
+    x[6] = cmul_x(x[6], cmul_tw<INV>(w4, w2));
+    x[7] = cmul_x(x[7], cmul_x(w4, w3));
+    x[8] = cmul_tw<INV>(x[8], w8);
+    x[9] = cmul_x(x[9], cmul_tw<INV>(w8, w1));
+    x[10] = cmul_x(x[10], cmul_tw<INV>(w8, w2));
+    x[11] = cmul_x(x[11], cmul_x(w8, w3));
+    x[12] = cmul_x(x[12], w12);
+    x[13] = cmul_x(x[13], cmul_tw<INV>(w12, w1));
+    x[14] = cmul_x(x[14], cmul_tw<INV>(w12, w2));
+    x[15] = cmul_x(x[15], cmul_x(w12, w3));
+  } else {
+    const float2* __restrict__ tp = tw + tw_offset<R>(NS) + bm;
+#pragma unroll
+    for (int r = 1; r < RP; ++r) {
+      float2 w = gldg(tp + r * NS);
+      if (INV) w.y = -w.y;
+      x[r] = cmul(x[r], w);
+    }
+  }
+}
+
+// Outputs r0, r0 + DR, .. of butterfly b of a pass with stride NS and radix RP
+// into the exchange buffer.
+template <int NS, int RP, int DR, int CNT>
+__device__ __forceinline__ void exchange_store(const float2 (&x)[CNT], float2* __restrict__ sb, int b, int r0) {
+  const int base = (b / NS) * (NS * RP) + (b & (NS - 1));
+  if constexpr (NS == 1 || NS % 16 == 0) {
+    // base + r stays inside one 16-entry block (NS = 1) or r * NS is a
+    // multiple of 16: the padded positions are pad(base) plus constants
+    float2* dst = sb + pad(base) + r0 * (NS + NS / 16);
+#pragma unroll
+    for (int k = 0; k < CNT; ++k) dst[k * DR * (NS + NS / 16)] = x[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < CNT; ++k) sb[pad(base + (r0 + k * DR) * NS)] = x[k];
+  }
+}
+
+// One radix-16 butterfly by two threads of 8 values each (R = 2 E): thread j
+// of T = N/8 holds the inputs r = h + 2 s of butterfly b = j % (N/16), h = j /
+// (N/16).  The first stage pairs r and r + 8, both the thread's own; then half
+// h = 0 goes on with the eight sums and h = 1 with the eight differences, each
+// a DFT of size 8, for which the two exchange four values by shuffles.  Every
+// value is rounded as in a whole butterfly's registers, so the results are
+// those of radix 16 bit for bit, with twice the threads per transform and an
+// exchange through shared memory less than in radix 8.
+// SCALED: the inputs are multiplied by g (scaled_butterfly).  On return a[k] is
+// output 2 k + h.
+template <int N, int NS, bool INV, bool SCALED>
+__device__ __forceinline__ void half_butterfly(float2 (&a)[8], const float (&g)[8], int b, int h,
+                                               const float2* __restrict__ tw) {
+  constexpr int LX = N / 16 < 16 ? N / 16 : 16;  // the partner's lane, see split_index
+  if constexpr (NS > 1) {
+    float2 w1, w2, w4, w8;
+    load_twiddles16<NS, INV>(tw, b & (NS - 1), w1, w2, w4, w8);
+    const float2 w3 = cmul_tw<INV>(w2, w1), w12 = cmul_tw<INV>(w8, w4);
+    // r = h + 2 s.  x q by cmul_x or, for INV and an even r, by cmul_y.
+    auto pick = [h](float2 odd, float2 even) { return h ? odd : even; };
+    auto mul = [h](float2 x, float2 q) {
+      float2 v = cmul_x(x, q);
+      if (INV) v.y = h ? v.y : cmul_y(x, q).y;
+      return v;
+    };
+    const float2 v = pick(w3, w2);
+    a[0] = pick(cmul_tw<INV>(a[0], w1), a[0]);
+    a[1] = mul(a[1], v);
+    a[2] = mul(a[2], pick(cmul_tw<INV>(w4, w1), w4));
+    a[3] = cmul_x(a[3], mul(w4, v));
+    a[4] = mul(a[4], pick(cmul_tw<INV>(w8, w1), w8));
+    a[5] = cmul_x(a[5], mul(w8, v));
+    a[6] = cmul_x(a[6], pick(cmul_tw<INV>(w12, w1), w12));
+    a[7] = cmul_x(a[7], mul(w12, v));
+  }
+  float2 e[8];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    float2 sum, dif;
+    if constexpr (SCALED) {
+      scaled_butterfly(a[s], g[s], a[s + 4], g[s + 4], h && s == 3, sum, dif);  // r = h + 2 s
+    } else {
+      sum = cadd(a[s], a[s + 4]);
+      dif = csub(a[s], a[s + 4]);
+    }
+    const float2 keep = h ? dif : sum, give = h ? sum : dif;
+    const float2 got = {__shfl_xor_sync(0xffffffffu, give.x, LX), __shfl_xor_sync(0xffffffffu, give.y, LX)};
+    e[2 * s] = h ? got : keep;
+    e[2 * s + 1] = h ? keep : got;
+  }
+#pragma unroll
+  for (int t = 1; t < 8; ++t) {
+    const float2 r = rot16<INV>(e[t], t);
+    e[t] = h ? r : e[t];
+  }
+  dft<8, INV>(e);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) a[k] = e[k];
+}
+
+// Thread of a transform that lane x of its T = N/8 lanes carries: the two
+// threads of a butterfly are N/16 apart, at N = 512 one warp; there the lanes
+// are dealt out so that they share one (lanes 0-15 and 16-31 still hold
+// neighbouring elements).
+template <int N>
+__device__ __forceinline__ int split_index(int x) {
+  static_assert(N <= 512, "two warps per transform at most");
+  if constexpr (N < 512)
+    return x;
+  else
+    return (x & 15) | ((x & 32) >> 1) | ((x & 16) << 1);
+}
+
+// One Stockham pass (stride NS) and, recursively, the remaining passes: R the
+// radix, E values per thread, E = R or (radix 16) R / 2.  SCALED: the first
+// pass takes its inputs times g.
+template <int N, int NS, bool INV, int E, int BAR, int R, bool SCALED>
+__device__ __forceinline__ void pass(float2 (&a)[E], const float (&g)[E], float2* __restrict__ sb, int j,
                                      const float2* __restrict__ tw) {
-  static_assert(E == 16 || E == 8 || E == N, "radix");
+  static_assert(E == R || (E == 8 && R == 16), "radix");
   constexpr int T = N / E;
   constexpr int REM = N / NS;
-  constexpr int RP = REM >= E ? E : REM;
-  constexpr int Q = E / RP;
+  constexpr int RP = REM >= R ? R : REM;
   constexpr bool LAST = (NS * RP == N);
+  if constexpr (RP > E) {
+    const int b = j & (N / 16 - 1), h = j / (N / 16);
+    half_butterfly<N, NS, INV, SCALED>(a, g, b, h, tw);
+    if constexpr (!LAST) exchange_store<NS, 16, 2>(a, sb, b, h);
+  } else {
+    constexpr int Q = E / RP;
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int b = j + q * T;
-    float2 x[RP];
+    for (int q = 0; q < Q; ++q) {
+      const int b = j + q * T;
+      float2 x[RP];
 #pragma unroll
-    for (int r = 0; r < RP; ++r) x[r] = a[q + r * Q];
-    if constexpr (NS > 1 && RP == 16) {
-      // W^r for r = 1..15 from the table's W^1, W^2, W^4, W^8 and at most two
-      // complex products each (a few ulps), so a radix-16 pass issues 4
-      // twiddle loads instead of 15
-      const int bm = b & (NS - 1);
-      const float2* __restrict__ tp = tw + tw_offset<E>(NS) + bm;
-      float2 w1 = gldg(tp + NS), w2 = gldg(tp + 2 * NS), w4 = gldg(tp + 4 * NS), w8 = gldg(tp + 8 * NS);
-      if (INV) {
-        w1.y = -w1.y;
-        w2.y = -w2.y;
-        w4.y = -w4.y;
-        w8.y = -w8.y;
-      }
-      const float2 w3 = cmul(w2, w1), w12 = cmul(w8, w4);
-      x[1] = cmul(x[1], w1);
-      x[2] = cmul(x[2], w2);
-      x[3] = cmul(x[3], w3);
-      x[4] = cmul(x[4], w4);
-      x[5] = cmul(x[5], cmul(w4, w1));
-      x[6] = cmul(x[6], cmul(w4, w2));
-      x[7] = cmul(x[7], cmul(w4, w3));
-      x[8] = cmul(x[8], w8);
-      x[9] = cmul(x[9], cmul(w8, w1));
-      x[10] = cmul(x[10], cmul(w8, w2));
-      x[11] = cmul(x[11], cmul(w8, w3));
-      x[12] = cmul(x[12], w12);
-      x[13] = cmul(x[13], cmul(w12, w1));
-      x[14] = cmul(x[14], cmul(w12, w2));
-      x[15] = cmul(x[15], cmul(w12, w3));
-    } else if constexpr (NS > 1) {
-      const int bm = b & (NS - 1);
-      const float2* __restrict__ tp = tw + tw_offset<E>(NS) + bm;
+      for (int r = 0; r < RP; ++r) x[r] = a[q + r * Q];
+      if constexpr (NS > 1) twiddle<NS, RP, R, INV>(x, b & (NS - 1), tw);
+      if constexpr (SCALED) {
 #pragma unroll
-      for (int r = 1; r < RP; ++r) {
-        float2 w = gldg(tp + r * NS);
-        if (INV) w.y = -w.y;
-        x[r] = cmul(x[r], w);
-      }
-    }
-    dft<RP, INV>(x);
-    if constexpr (LAST) {
-#pragma unroll
-      for (int r = 0; r < RP; ++r) a[q + r * Q] = x[r];
-    } else {
-      const int base = (b / NS) * (NS * RP) + (b & (NS - 1));
-      if constexpr (NS == 1 || NS % 16 == 0) {
-        // base + r stays inside one 16-entry block (NS = 1) or r * NS is a
-        // multiple of 16: the padded positions are pad(base) plus constants
-        float2* dst = sb + pad(base);
-#pragma unroll
-        for (int r = 0; r < RP; ++r) dst[r * (NS + NS / 16)] = x[r];
+        for (int t = 0; t < RP / 2; ++t) {
+          float2 sum, dif;
+          scaled_butterfly(x[t], g[q + t * Q], x[t + RP / 2], g[q + (t + RP / 2) * Q], t == RP / 2 - 1, sum, dif);
+          x[t] = sum;
+          x[t + RP / 2] = rot16<INV>(dif, t * (16 / RP));
+        }
+        dft<RP, INV, RP / 2>(x);
       } else {
+        dft<RP, INV>(x);
+      }
+      if constexpr (LAST) {
 #pragma unroll
-        for (int r = 0; r < RP; ++r) sb[pad(base + r * NS)] = x[r];
+        for (int r = 0; r < RP; ++r) a[q + r * Q] = x[r];
+      } else {
+        exchange_store<NS, RP, 1>(x, sb, b, 0);
       }
     }
   }
@@ -280,18 +428,25 @@ __device__ __forceinline__ void pass(float2 (&a)[E], float2* __restrict__ sb, in
     group_sync<BAR, T>();
     load_strided<T, E>(a, sb, j);
     group_sync<BAR, T>();
-    pass<N, NS * RP, INV, E, BAR>(a, sb, j, tw);
+    pass<N, NS * RP, INV, E, BAR, R, false>(a, g, sb, j, tw);
   }
 }
 
-// Full FFT of length N (unnormalised; INV uses exp(+2 pi i ...)) in radix E,
-// with `tw` the radix-E tables.  Every thread of the CTA (BAR = 0), or of the
-// N/E-thread group synchronised by BAR, must call it: it synchronises those
-// threads between passes, the last time after their last read of the exchange
-// buffer, which is free for reuse on return.
-template <int N, bool INV, int E, int BAR = 0>
+// Full FFT of length N (unnormalised; INV uses exp(+2 pi i ...)) in radix R
+// with E values per thread, `tw` the radix-R tables.  Every thread of the CTA
+// (BAR = 0), or of the N/E-thread group synchronised by BAR, must call it (at
+// E < R every lane of the warp): it synchronises those threads between passes,
+// the last time after their last read of the exchange buffer, which is free
+// for reuse on return.  block_fft_scaled transforms a[s] * g[s].
+template <int N, bool INV, int E, int BAR = 0, int R = E>
 __device__ __forceinline__ void block_fft(float2 (&a)[E], float2* sb, int j, const float2* __restrict__ tw) {
-  pass<N, 1, INV, E, BAR>(a, sb, j, tw);
+  const float none[E] = {};
+  pass<N, 1, INV, E, BAR, R, false>(a, none, sb, j, tw);
+}
+template <int N, bool INV, int E, int BAR = 0, int R = E>
+__device__ __forceinline__ void block_fft_scaled(float2 (&a)[E], const float (&g)[E], float2* sb, int j,
+                                                 const float2* __restrict__ tw) {
+  pass<N, 1, INV, E, BAR, R, true>(a, g, sb, j, tw);
 }
 
 }  // namespace fft

@@ -38,7 +38,7 @@ __host__ __device__ constexpr int fft_bar() {
 // transform a copy of the last pair in their own buffer and store nothing,
 // so every thread reaches the transform's barriers.  COH: L2-only loads of
 // data other CTAs of the same launch wrote.
-template <int N, int E, bool COH = false>
+template <int N, int E, int R = E, bool COH = false>
 __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, float2* __restrict__ spec,
                                               const float2* __restrict__ tw, int j, int pp, int P, int bx) {
   constexpr int T = N / E;
@@ -57,7 +57,7 @@ __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, flo
 #pragma unroll
   for (int s = 0; s < E; ++s)
     a[s] = make_float2(gldstream<COH>(ra + j + s * T), gldstream<COH>(rb + j + s * T));
-  fft::block_fft<N, false, E, BAR>(a, sb, j, tw);
+  fft::block_fft<N, false, E, BAR, R>(a, sb, j, tw);
   fft::store_strided<T, E>(a, sb, j);
   __syncthreads();
 
@@ -103,7 +103,7 @@ __device__ __forceinline__ float poisson_mult(float k2x, float k2y, float scale)
 
 // Transform thread j of spectrum row y of a CTA carrying KB rows, rows
 // [bx * KB, +KB) (blockDim = (T, KB): j = threadIdx.x, y = threadIdx.y).
-template <int N, int E, bool COH = false>
+template <int N, int E, int R = E, bool COH = false>
 __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float2* __restrict__ tw,
                                           const float* __restrict__ k2, float scale, int j, int y, int KB,
                                           int bx) {
@@ -121,17 +121,21 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
   float2 a[E];
 #pragma unroll
   for (int s = 0; s < E; ++s) a[s] = gldstream<COH>(row + j + s * T);
-  fft::block_fft<N, false, E, BAR>(a, sb, j, tw);
+  fft::block_fft<N, false, E, BAR, R>(a, sb, j, tw);
 
   const float k2y = gldg(k2 + ky);
+  float g[E];
 #pragma unroll
-  for (int s = 0; s < E; ++s) {
-    const float g = poisson_mult<(N < 8192)>(gldg(k2 + j + s * T), k2y, scale);
-    // (the products fuse into the inverse transform's first butterflies: 39.6
-    // against 43.0 us at N = 4096)
-    a[s] = make_float2(a[s].x * g, a[s].y * g);
+  for (int s = 0; s < E; ++s) g[s] = poisson_mult<(N < 8192)>(gldg(k2 + j + s * T), k2y, scale);
+  if constexpr (N < 2048) {
+    fft::block_fft_scaled<N, true, E, BAR, R>(a, g, sb, j, tw);
+  } else {
+    // the products fuse into the first butterflies: 39.6 against 43.0 us at N =
+    // 4096
+#pragma unroll
+    for (int s = 0; s < E; ++s) a[s] = make_float2(a[s].x * g[s], a[s].y * g[s]);
+    fft::block_fft<N, true, E, BAR, R>(a, sb, j, tw);
   }
-  fft::block_fft<N, true, E, BAR>(a, sb, j, tw);
   __syncthreads();  // rows clamped to N/2 were loaded by other threads
   if (kreq <= H) {
 #pragma unroll
@@ -142,7 +146,7 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
 // ---------------------------------------------------------------- rows inv --
 // Thread layout as for rows_fwd_body; the extra threads of a persistent CTA
 // (pp >= P) transform their own buffer and store nothing.
-template <int N, int E, bool COH = false>
+template <int N, int E, int R = E, bool COH = false>
 __device__ __forceinline__ void rows_inv_body(const float2* __restrict__ spec, float* __restrict__ p,
                                               const float2* __restrict__ tw, int j, int pp, int P, int bx) {
   constexpr int T = N / E;
@@ -196,7 +200,7 @@ __device__ __forceinline__ void rows_inv_body(const float2* __restrict__ spec, f
   float2 a[E];
   fft::load_strided<T, E>(a, sb, j);
   fft::group_sync<BAR, T>();
-  fft::block_fft<N, true, E, BAR>(a, sb, j, tw);
+  fft::block_fft<N, true, E, BAR, R>(a, sb, j, tw);
   if (COH && pp >= P) return;
   float* ra = p + (size_t)(i0 + 2 * pp) * N;
   float* rb = ra + N;

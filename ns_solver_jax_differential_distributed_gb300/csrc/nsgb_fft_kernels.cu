@@ -36,107 +36,144 @@ template <int N, int E>
 constexpr bool cols_two() {
   return E == 8 || N >= 8192;
 }
-template <int N, int E>
+template <int N, int E, int R>
+__device__ __forceinline__ int cols_thread() {
+  if constexpr (E < R)
+    return fft::split_index<N>(threadIdx.x);
+  else
+    return threadIdx.x;
+}
+template <int N, int E, int R>
 __global__ void __launch_bounds__(1024) k_rows_fwd(const float* __restrict__ rhs, float2* __restrict__ spec,
                                                    const float2* __restrict__ tw) {
-  rows_fwd_body<N, E>(rhs, spec, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
+  rows_fwd_body<N, E, R>(rhs, spec, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
 }
-template <int N, int E>
+template <int N, int E, int R>
 __global__ void __launch_bounds__(cols_two<N, E>() ? 512 : 768, cols_two<N, E>() ? 2 : 1) k_cols(float2* __restrict__ spec,
                                                               const float2* __restrict__ tw,
                                                               const float* __restrict__ k2, float scale) {
-  cols_body<N, E>(spec, tw, k2, scale, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
+  cols_body<N, E, R>(spec, tw, k2, scale, cols_thread<N, E, R>(), threadIdx.y, blockDim.y, blockIdx.x);
 }
-template <int N, int E>
+template <int N, int E, int R>
 __global__ void __launch_bounds__(1024) k_rows_inv(const float2* __restrict__ spec, float* __restrict__ p,
                                                    const float2* __restrict__ tw) {
-  rows_inv_body<N, E>(spec, p, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
+  rows_inv_body<N, E, R>(spec, p, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
 }
 // Ensemble variants: blockIdx.y selects the member.
-template <int N, int E>
+template <int N, int E, int R>
 __global__ void __launch_bounds__(1024) k_rows_fwd_b(const SolveDev* __restrict__ sv,
                                                      const float2* __restrict__ tw) {
   const FftPtrs f = sv[blockIdx.y].fft;
-  rows_fwd_body<N, E>(f.rhs, f.spec, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
+  rows_fwd_body<N, E, R>(f.rhs, f.spec, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
 }
-template <int N, int E>
+template <int N, int E, int R>
 __global__ void __launch_bounds__(cols_two<N, E>() ? 512 : 768, cols_two<N, E>() ? 2 : 1) k_cols_b(const SolveDev* __restrict__ sv,
                                                                 const float2* __restrict__ tw,
                                                                 const float* __restrict__ k2, float scale) {
-  cols_body<N, E>(sv[blockIdx.y].fft.spec, tw, k2, scale, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
+  cols_body<N, E, R>(sv[blockIdx.y].fft.spec, tw, k2, scale, cols_thread<N, E, R>(), threadIdx.y, blockDim.y, blockIdx.x);
 }
-template <int N, int E>
+template <int N, int E, int R>
 __global__ void __launch_bounds__(1024) k_rows_inv_b(const SolveDev* __restrict__ sv,
                                                      const float2* __restrict__ tw) {
   const FftPtrs f = sv[blockIdx.y].fft;
-  rows_inv_body<N, E>(f.spec, f.p, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
+  rows_inv_body<N, E, R>(f.spec, f.p, tw, threadIdx.x, threadIdx.y, blockDim.y, blockIdx.x);
 }
 
 // ------------------------------------------------------------- launchers --
-template <int N, int E>
-static const float2* radix_tables(const FftLaunch& L) {
-  return L.tw + (E == 8 ? fft::tw8_offset(N) : 0);
+// Radix-16 passes by threads of 8 values (fft::half_butterfly) where a step
+// waits for the transforms' latency: the same bits from twice the threads.  Step
+// with whole / split butterflies, us: N = 16 8.7 / 7.5, 256 11.6 / 10.3 (rows
+// alone or columns alone 10.9; a batch of 8 15.7 / 14.1, of 30 29.2 / 30.4), 512,
+// columns only, 14.2 / 13.4 (batch of 11 39.7 / 41.1); from N = 1024 on it waits
+// for shared memory.  CTAs too large for twice the threads keep whole ones.
+constexpr int kSplitRowsN = 256, kSplitColsN = 512;
+template <int N>
+static bool rows_split(const FftLaunch& L) {
+  return N <= kSplitRowsN && L.radix_rows == 16 && L.rows_per_cta / 2 * (N / 8) <= 1024;
+}
+template <int N>
+static bool cols_split(const FftLaunch& L) {
+  return N <= kSplitColsN && L.radix_cols == 16 && L.cols_per_cta * (N / 8) <= 512;
 }
 
+template <int N, int R>
+static const float2* radix_tables(const FftLaunch& L) {
+  return L.tw + (R == 8 ? fft::tw8_offset(N) : 0);
+}
 
-template <int N, int E>
+template <int N, int E, int R>
 static cudaError_t stage_rows_fwd(const FftLaunch& L, const SolveDev* sv, int count, cudaStream_t st) {
   constexpr int T = N / E;
   const int P = L.rows_per_cta / 2;
   const size_t smem = (size_t)P * pair_stride<N>() * sizeof(float2);
   if (smem > 48 * 1024) {
-    const cudaError_t e = raise_smem_limit(sv ? (const void*)k_rows_fwd_b<N, E> : (const void*)k_rows_fwd<N, E>);
+    const cudaError_t e = raise_smem_limit(sv ? (const void*)k_rows_fwd_b<N, E, R> : (const void*)k_rows_fwd<N, E, R>);
     if (e != cudaSuccess) return e;
   }
   if (sv)
-    k_rows_fwd_b<N, E><<<dim3(N / (2 * P), count), dim3(T, P), smem, st>>>(sv, radix_tables<N, E>(L));
+    k_rows_fwd_b<N, E, R><<<dim3(N / (2 * P), count), dim3(T, P), smem, st>>>(sv, radix_tables<N, R>(L));
   else
-    k_rows_fwd<N, E><<<N / (2 * P), dim3(T, P), smem, st>>>(L.rhs, L.spec, radix_tables<N, E>(L));
+    k_rows_fwd<N, E, R><<<N / (2 * P), dim3(T, P), smem, st>>>(L.rhs, L.spec, radix_tables<N, R>(L));
   return cudaGetLastError();
 }
 
-template <int N, int E>
+template <int N, int E, int R>
 static cudaError_t stage_cols(const FftLaunch& L, const SolveDev* sv, int count, cudaStream_t st) {
   constexpr int T = N / E;
   const int KB = L.cols_per_cta;
   const size_t smem = (size_t)KB * pair_stride<N>() * sizeof(float2);
   if (smem > 48 * 1024) {
-    const cudaError_t e = raise_smem_limit(sv ? (const void*)k_cols_b<N, E> : (const void*)k_cols<N, E>);
+    const cudaError_t e = raise_smem_limit(sv ? (const void*)k_cols_b<N, E, R> : (const void*)k_cols<N, E, R>);
     if (e != cudaSuccess) return e;
   }
   if (sv)
-    k_cols_b<N, E><<<dim3((N / 2) / KB + 1, count), dim3(T, KB), smem, st>>>(sv, radix_tables<N, E>(L), L.k2,
+    k_cols_b<N, E, R><<<dim3((N / 2) / KB + 1, count), dim3(T, KB), smem, st>>>(sv, radix_tables<N, R>(L), L.k2,
                                                                             L.scale);
   else
-    k_cols<N, E><<<(N / 2) / KB + 1, dim3(T, KB), smem, st>>>(L.spec, radix_tables<N, E>(L), L.k2, L.scale);
+    k_cols<N, E, R><<<(N / 2) / KB + 1, dim3(T, KB), smem, st>>>(L.spec, radix_tables<N, R>(L), L.k2, L.scale);
   return cudaGetLastError();
 }
 
-template <int N, int E>
+template <int N, int E, int R>
 static cudaError_t stage_rows_inv(const FftLaunch& L, const SolveDev* sv, int count, cudaStream_t st) {
   constexpr int T = N / E;
   const int P = L.rows_per_cta / 2;
   const size_t smem = (size_t)P * pair_stride<N>() * sizeof(float2);
   if (smem > 48 * 1024) {
-    const cudaError_t e = raise_smem_limit(sv ? (const void*)k_rows_inv_b<N, E> : (const void*)k_rows_inv<N, E>);
+    const cudaError_t e = raise_smem_limit(sv ? (const void*)k_rows_inv_b<N, E, R> : (const void*)k_rows_inv<N, E, R>);
     if (e != cudaSuccess) return e;
   }
   if (sv)
-    k_rows_inv_b<N, E><<<dim3(N / (2 * P), count), dim3(T, P), smem, st>>>(sv, radix_tables<N, E>(L));
+    k_rows_inv_b<N, E, R><<<dim3(N / (2 * P), count), dim3(T, P), smem, st>>>(sv, radix_tables<N, R>(L));
   else
-    k_rows_inv<N, E><<<N / (2 * P), dim3(T, P), smem, st>>>(L.spec, L.p, radix_tables<N, E>(L));
+    k_rows_inv<N, E, R><<<N / (2 * P), dim3(T, P), smem, st>>>(L.spec, L.p, radix_tables<N, R>(L));
   return cudaGetLastError();
 }
 
 template <int N>
 static cudaError_t launch_poisson_fft(const FftLaunch& L, const SolveDev* sv, int count, cudaStream_t st) {
-  const bool r8 = L.radix_rows == 8, c8 = L.radix_cols == 8;
+  constexpr int E = fft::ept(N);
+  const int r = rows_split<N>(L) ? 1 : L.radix_rows == 8 ? 2 : 0;
+  const int c = cols_split<N>(L) ? 1 : L.radix_cols == 8 ? 2 : 0;
   cudaError_t e = cudaSuccess;
-  if (sv || L.rhs) e = r8 ? stage_rows_fwd<N, 8>(L, sv, count, st) : stage_rows_fwd<N, fft::ept(N)>(L, sv, count, st);
-  if (e == cudaSuccess && (sv || L.do_cols))
-    e = c8 ? stage_cols<N, 8>(L, sv, count, st) : stage_cols<N, fft::ept(N)>(L, sv, count, st);
-  if (e == cudaSuccess && (sv || L.p))
-    e = r8 ? stage_rows_inv<N, 8>(L, sv, count, st) : stage_rows_inv<N, fft::ept(N)>(L, sv, count, st);
+  if (sv || L.rhs) {
+    if constexpr (N <= kSplitRowsN)
+      if (r == 1) e = stage_rows_fwd<N, 8, 16>(L, sv, count, st);
+    if (r == 2) e = stage_rows_fwd<N, 8, 8>(L, sv, count, st);
+    if (r == 0) e = stage_rows_fwd<N, E, 16>(L, sv, count, st);
+  }
+  if (e == cudaSuccess && (sv || L.do_cols)) {
+    if constexpr (N <= kSplitColsN)
+      if (c == 1) e = stage_cols<N, 8, 16>(L, sv, count, st);
+    if (c == 2) e = stage_cols<N, 8, 8>(L, sv, count, st);
+    if (c == 0) e = stage_cols<N, E, 16>(L, sv, count, st);
+  }
+  if (e == cudaSuccess && (sv || L.p)) {
+    if constexpr (N <= kSplitRowsN)
+      if (r == 1) e = stage_rows_inv<N, 8, 16>(L, sv, count, st);
+    if (r == 2) e = stage_rows_inv<N, 8, 8>(L, sv, count, st);
+    if (r == 0) e = stage_rows_inv<N, E, 16>(L, sv, count, st);
+  }
   return e;
 }
 

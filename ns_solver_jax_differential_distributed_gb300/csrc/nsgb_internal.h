@@ -22,14 +22,6 @@ struct FftLaunch {
   int radix_rows = 16;         // Stockham radix of the row passes (16 or 8)
   int radix_cols = 16;         // ... and of the column pass
 };
-// Radix of the row and column passes of a plan that is not tuned: 8 where a
-// step waits for the transforms' latency (twice the threads share a transform),
-// 16 where it waits for shared memory (fewer exchanges).  Measured, step in
-// radix 16 / 8: N = 16 8.4 / 7.2 us, 256 10.8 / 9.4 (a batch of 8 15.0 / 13.9, of
-// 15 19.3 / 19.4, of 30 28.7 / 30.0), 512 13.6 / 11.3 but a batch of 11 39.3 /
-// 42.4: there radix 8 in the columns only, 12.6 and 39.9; 1024 20.1 / 20.5.
-inline int fft_default_radix_rows(int N) { return N <= 256 ? 8 : 16; }
-inline int fft_default_radix_cols(int N) { return N <= 512 ? 8 : 16; }
 cudaError_t poisson_fft(int N, const FftLaunch& L, cudaStream_t st);
 size_t fft_rows_smem_bytes(int N, int rows_per_cta);
 size_t fft_cols_smem_bytes(int N, int cols_per_cta);
@@ -195,7 +187,7 @@ cudaError_t launch_gsum(const double* gpart, int nblk, int theta_len, float* dJ,
 struct alignas(16) ResidentArgs {
   StepConsts c;
   int scheme = 0;
-  const float2* tw = nullptr;  // twiddles of the resident radix
+  const float2* tw = nullptr;  // radix-16 twiddles
   const float* k2 = nullptr;
   float scale = 0.f;
   const float* theta = nullptr;
@@ -219,7 +211,7 @@ struct alignas(16) ResidentArgs {
   double* gpart = nullptr;     // theta sensitivities, [tile][3]
   float* dJdu0 = nullptr;      // optional
 };
-int resident_radix(int N);        // radix of its transforms, 0: no instance for N
+bool resident_size(int N);        // whether it has an instance for N (radix-16 transforms)
 cudaError_t launch_resident(int N, const ResidentArgs& a, cudaStream_t st);
 // Gradient solves of one scheme, one cluster each, in one launch: tab is a
 // device table of their arguments.

@@ -141,8 +141,6 @@ extern "C" int nsgb_poisson_noalloc(int N, double L, const float* rhs, float* p,
   Lc.scale = scale;
   Lc.rows_per_cta = N >= 1024 ? 4 : 8;
   Lc.cols_per_cta = 1;
-  Lc.radix_rows = nsgb::fft_default_radix_rows(N);  // a plan's
-  Lc.radix_cols = nsgb::fft_default_radix_cols(N);
   e = nsgb::poisson_fft(N, Lc, st);
   if (e != cudaSuccess) return fail(NSGB_ERR_CUDA, "poisson kernels: %s", cudaGetErrorString(e));
   return nsgb::finish_call(st);

@@ -5,14 +5,16 @@
 // Up to N = 128 a step's four launches cost more than their work.  Here C CTAs,
 // one cluster, own R = N / C rows each and keep the state (u* or lambda, the
 // pressure, and the spectrum's pieces) in shared memory for all steps.
-// Measured per step against four launches in a graph: N = 32 3.1 / 7.8 us, 64
-// 3.1 / 8.0, 128 4.8 / 8.9; with the gradient, every state kept, 7.7 / 15.8, 7.7 /
-// 15.9, 11.3 / 17.9.  At N = 256 sixteen CTAs have too many cells each (10.0 / 10.4
-// and 24 / 21 us), so the four launches stay.  What bounds a step is latency:
-// three cluster barriers of about 0.35 us and four transforms of a few warps
-// of about 0.5 us; so transforms are of radix 8 (radix 16 on half the threads
-// took 9.4 us per step at N = 128), cells go four to a thread, and the
-// objective and theta sums run in the warps that the row transforms leave
+// Measured per step against four launches in a graph: N = 32 3.6 / 8.7 us, 64
+// 3.5 / 8.5, 128 4.4 / 9.0; with the gradient, every state kept, 8.5 / 17.4, 8.4 /
+// 17.7, 10.8 / 17.7.  At N = 256 sixteen CTAs have too many cells each (9.9 / 9.6
+// and 24 / 19.6 us), so the four launches stay; N = 16 is less than one 32-wide
+// tile of the sums below.  What bounds a step is latency: three cluster barriers
+// of about 0.35 us and four transforms of a few warps of about 0.5 us; so two
+// threads share a radix-16 butterfly (fft::half_butterfly; whole ones on half
+// the threads took 9.4 us per step at N = 128, radix 8 5.2 against 4.6 and at N =
+// 64 3.4 against 3.6), cells go four to a thread, and the objective and theta
+// sums run in the warps that the row transforms leave
 // idle.  A step is three phases between cluster barriers:
 //   1. stencil of the own rows (halo rows are kept beside them), right-hand
 //      side, forward row transforms, split into the two rows' half spectra and
@@ -25,8 +27,8 @@
 // need no residency check and no polling.
 //
 // The arithmetic is that of the batched kernels at the default 32 x 8 tiles,
-// value for value: the same cell functions, the transforms of the plan's
-// radix, objective and theta partials summed per 32 x 8 tile in the same
+// value for value: the same cell functions, the same radix-16 transforms,
+// objective and theta partials summed per 32 x 8 tile in the same
 // order, so a resident solve, an ensemble member and a batched gradient give
 // the same bits.
 #include <type_traits>
@@ -40,7 +42,7 @@ namespace res {
 
 constexpr int kTileW = 32, kTileH = 8;  // tiles of the objective and theta partials
 
-// R rows per CTA of N x N, transforms of radix E.
+// R rows per CTA of N x N, radix-16 transforms with E values per thread.
 template <int N, int R, int E>
 struct Lay {
   static constexpr int M = N - 1, H = N / 2;
@@ -332,7 +334,7 @@ struct Solve {
       float2* sb = X + y * L::PS;
       fft::load_strided<T, E>(v, sb, j);
       __syncwarp();
-      fft::block_fft<N, false, E, -1>(v, sb, j, a.tw);
+      fft::block_fft<N, false, E, -1, 16>(v, sb, j, a.tw);
       fft::store_strided<T, E>(v, sb, j);
     } else {
       sums<KIND>(PR * T / 32);
@@ -357,14 +359,12 @@ struct Solve {
 #pragma unroll
       for (int s = 0; s < E; ++s) v[s] = ci[j + s * T];
       float2* sb = X + y * L::PS;
-      fft::block_fft<N, false, E, -1>(v, sb, j, a.tw);
+      fft::block_fft<N, false, E, -1, 16>(v, sb, j, a.tw);
       const float k2y = gldg(a.k2 + (valid ? k : H));
+      float g[E];
 #pragma unroll
-      for (int s = 0; s < E; ++s) {
-        const float g = poisson_mult<true>(gldg(a.k2 + j + s * T), k2y, a.scale);
-        v[s] = make_float2(v[s].x * g, v[s].y * g);
-      }
-      fft::block_fft<N, true, E, -1>(v, sb, j, a.tw);
+      for (int s = 0; s < E; ++s) g[s] = poisson_mult<true>(gldg(a.k2 + j + s * T), k2y, a.scale);
+      fft::block_fft_scaled<N, true, E, -1, 16>(v, g, sb, j, a.tw);
       if (valid) {
 #pragma unroll
         for (int s = 0; s < E; ++s) {
@@ -390,7 +390,7 @@ struct Solve {
                : m < H            ? make_float2(w.x - w.w, w.y + w.z)
                                   : make_float2(w.x + w.w, w.z - w.y);
       }
-      fft::block_fft<N, true, E, -1>(v, X + y * L::PS, j, a.tw);
+      fft::block_fft<N, true, E, -1, 16>(v, X + y * L::PS, j, a.tw);
 #pragma unroll
       for (int s = 0; s < E; ++s) {
         P[(2 * y + 3) * N + j + s * T] = v[s].x;
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(Lay<N, R, E>::NT, 1) k_resident_batch(const Re
 
 }  // namespace res
 
-// Rows per CTA and radix of the resident kernel's instances.
+// Rows per CTA and values per transform thread of the resident kernel's instances.
 #ifndef NSGB_RESIDENT
 #define NSGB_RESIDENT(X) X(32, 16, 8) X(64, 8, 8) X(128, 8, 8)
 #endif
@@ -749,11 +749,11 @@ static cudaError_t launch_resident_batch_t(const ResidentArgs* tab, int count, c
   return cudaLaunchKernelEx(&cfg, res::k_resident_batch<N, R, E, SCHEME>, tab);
 }
 
-int resident_radix(int N) {
-#define NSGB_RESIDENT_CASE(NN, R, E) if (N == NN) return E;
+bool resident_size(int N) {
+#define NSGB_RESIDENT_CASE(NN, R, E) if (N == NN) return true;
   NSGB_RESIDENT(NSGB_RESIDENT_CASE)
 #undef NSGB_RESIDENT_CASE
-  return 0;
+  return false;
 }
 
 template <int N, int R, int E, int SCHEME>
