@@ -249,8 +249,8 @@ struct Carver {
 };
 
 struct RolloutWs {
-  float *usA, *usB, *p, *rhs, *spec, *spec2, *jpart;
-  double* jsteps;
+  float *usA, *usB, *p, *rhs, *spec, *spec2;
+  double *jpart, *jsteps;
   int* ctr;
   float* theta;  // the call's theta, at a fixed place for captured graphs
   int steps;  // rows of jpart
@@ -282,7 +282,7 @@ RolloutWs carve_rollout(const nsgb_plan* plan, int steps, void* ws) {
   w.rhs = cv.take<float>(NN);
   w.spec = cv.take<float>(spec_floats(plan->N));
   w.spec2 = cv.take<float>(spec_floats(plan->N));
-  w.jpart = cv.take<float>((size_t)(steps > 0 ? steps : 1) * nblk);
+  w.jpart = cv.take<double>((size_t)(steps > 0 ? steps : 1) * nblk);
   w.jsteps = cv.take<double>(steps > 0 ? steps : 1);
   w.steps = steps > 0 ? steps : 1;
   w.bytes = cv.off;
@@ -2250,7 +2250,7 @@ PersLayout pers_layout(const nsgb_member* m, int count) {
     P.jpart_off[k] = off;
     int tw, th;
     pers_tile(m[k].plan->N, tw, th);
-    off += align_up(sizeof(float) * (size_t)m[k].total_steps * stencil_nblocks(m[k].plan->N, tw, th));
+    off += align_up(sizeof(double) * (size_t)m[k].total_steps * stencil_nblocks(m[k].plan->N, tw, th));
   }
   P.bytes = off;
   return P;
@@ -2299,7 +2299,7 @@ int nsgb_ensemble_persistent(const nsgb_member* members_in, int count, void* wor
     const nsgb_member& x = members[i];
     void* state = x.state ? x.state : (void*)(base + P.ens.state_off[i]);
     tab[k] = make_solvedev(x, state);
-    float* jp = (float*)(base + P.jpart_off[i]);
+    double* jp = (double*)(base + P.jpart_off[i]);
     for (auto& a : tab[k].st) {
       a.jpart = jp;
       a.jpart_rows = steps;

@@ -342,7 +342,7 @@ __device__ __forceinline__ void fused_rows_body(const FusedArgs& fa) {
         const size_t o = (size_t)((t - 2) & M) * N + col;
         st4_stream(uso_x, o, sx2);
         st4_stream(uso_y, o, sy2);
-        jacc.add(u2x, sF[t - r0 - 1], t);
+        jacc.add(u2x, sF[t - r0 - 1]);
         if (h == 0) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) rhe[kk] = rh[kk];
@@ -448,7 +448,8 @@ __device__ __forceinline__ void fused_rows_body(const FusedArgs& fa) {
   fft::group_sync<1, ST>();
   if (warp == 0) {
     const DFloat z = {0.f, 0.f};
-    const float v = warp_sum_df(lane < NWS ? sRed[lane] : z).hi;
+    const DFloat w = warp_sum_df(lane < NWS ? sRed[lane] : z);
+    const double v = (double)w.hi + (double)w.lo;
     if (lane == 0 && (unsigned)step < (unsigned)a.jpart_rows) {
       const int nblk = gridDim.x * gridDim.y;
       gst(a.jpart + (size_t)step * nblk + blockIdx.y * gridDim.x + blockIdx.x, v);

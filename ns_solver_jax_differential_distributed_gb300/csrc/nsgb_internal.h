@@ -39,7 +39,7 @@ struct StencilArgs {
   float* us_out = nullptr;       // (2,N,N) next u*
   float* rhs = nullptr;          // (N,N) div(u*)/dt
   float* u_out = nullptr;        // optional (2,N,N): the projected state u^n
-  float* jpart = nullptr;        // per-block partial sums of u_x * f_x, [step][nblk]
+  double* jpart = nullptr;       // per-block partial sums of u_x * f_x, [step][nblk]
   int jpart_rows = 0;            // rows allocated in jpart (a store beyond is skipped)
   const float* theta = nullptr;  // device theta
   int theta_len = 2;
@@ -137,7 +137,7 @@ cudaError_t launch_ensemble_poison(const unsigned* bar, const SolveDev* dev, int
 cudaError_t launch_project(const float* us, const float* p, float* u_out, const StepConsts& c,
                            cudaStream_t st);
 // Sum the per-block partials of each step in a fixed order and accumulate J.
-cudaError_t launch_jreduce(const float* jpart, int nblk, int steps, double* jsteps, float* J,
+cudaError_t launch_jreduce(const double* jpart, int nblk, int steps, double* jsteps, float* J,
                            double jscale, cudaStream_t st);
 // *step_ctr = value (add = false) or *step_ctr += value (add = true)
 cudaError_t launch_step_counter(int* step_ctr, int value, bool add, cudaStream_t st);
@@ -202,7 +202,7 @@ struct alignas(16) ResidentArgs {
   int t_from_step = 1;         // forcing time step * dt, or t_fixed (a single step)
   float t_fixed = 0.f;
   const float* u0 = nullptr;
-  float* jpart = nullptr;      // objective partials, [step][tile]
+  double* jpart = nullptr;     // objective partials, [step][tile]
   float* u_final = nullptr;    // optional
   float* ckpt = nullptr;       // checkpoints every `every` steps (nullptr: a plain rollout)
   float* ustore = nullptr;     // a segment's states

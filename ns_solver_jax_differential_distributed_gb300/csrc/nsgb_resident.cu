@@ -307,7 +307,7 @@ struct Solve {
       const int ty = t / S, tx = t % S;
       const float* v = sm + L::J_OFF + ty * kTileH * S + tx;
       const float s = ((v[0] + v[4 * S]) + (v[2 * S] + v[6 * S])) + ((v[S] + v[5 * S]) + (v[3 * S] + v[7 * S]));
-      gst(a.jpart + (size_t)jstep * (N / kTileH * S) + (r0 / kTileH + ty) * S + tx, s);
+      gst(a.jpart + (size_t)jstep * (N / kTileH * S) + (r0 / kTileH + ty) * S + tx, (double)s);
     }
     if (KIND == kTheta && t < (R / kTileH) * S * 3) {
       const int comp = t % 3, tile = t / 3, ty = tile / S, tx = tile % S;

@@ -133,23 +133,24 @@ __device__ __forceinline__ void ld4s(const float* s, float (&o)[4]) {
   o[3] = v.w;
 }
 
-// A thread's objective partial sum u f over its cells of a band: float over up
-// to 16 rows (iteration index t), double-float over the band (a float sum down
-// a tall band loses digits of an objective whose terms cancel).  The step
-// kernel at N = 4096, bands of 1024 x 54, central: 70.1 us; 69.6 us with a
-// float sum, 71.9 us adding every row in double-float.
+// A thread's objective partial sum u f over its cells of a band: the four
+// cells of a row in float, as a tile's thread has them, then every row's sum
+// in double-float: hi by Knuth's TwoSum, the rounding errors in lo (a float sum
+// down a tall band loses digits of an objective whose terms cancel).  Error over
+// the summed magnitudes at N = 4096 1.0e-9 with a float sum over 16 rows, 1.7e-11
+// so (3.1e-10 with tiles of 64 x 16); a step 172.2 -> 173.1 us.
 struct ObjectiveSum {
   DFloat acc = {0.f, 0.f};
-  float s = 0.f;
-  __device__ __forceinline__ void add(const float (&u)[4], float f, int t) {
+  __device__ __forceinline__ void add(const float (&u)[4], float f) {
+    float v = fmul(u[0], f);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) s = __fmaf_rn(u[k], f, s);
-    if ((t & 15) == 15) {
-      acc = df_add(acc, {s, 0.f});
-      s = 0.f;
-    }
+    for (int k = 1; k < 4; ++k) v = __fmaf_rn(u[k], f, v);
+    const float s = __fadd_rn(acc.hi, v);
+    const float b = __fsub_rn(s, acc.hi);
+    acc.lo = __fadd_rn(acc.lo, __fadd_rn(__fsub_rn(acc.hi, __fsub_rn(s, b)), __fsub_rn(v, b)));
+    acc.hi = s;
   }
-  __device__ __forceinline__ DFloat total() const { return df_add(acc, {s, 0.f}); }
+  __device__ __forceinline__ DFloat total() const { return acc; }
 };
 
 // Copy one band row (W + 8 columns, or the wrapped row when W = N) of `field`

@@ -282,7 +282,7 @@ __device__ __forceinline__ void stencil_rows_body(const StencilArgs& a, int step
           st4(a.u_out, o, u2x);
           st4(a.u_out + NN, o, u2y);
         }
-        jacc.add(u2x, sF[t - r0 - 1], t);
+        jacc.add(u2x, sF[t - r0 - 1]);
       }
     }
 
@@ -334,7 +334,8 @@ __device__ __forceinline__ void stencil_rows_body(const StencilArgs& a, int step
   __syncthreads();
   if (warp == 0) {
     const DFloat z = {0.f, 0.f};
-    float v = warp_sum_df(lane < nwarps ? sRed[lane] : z).hi;
+    const DFloat w = warp_sum_df(lane < nwarps ? sRed[lane] : z);
+    double v = (double)w.hi + (double)w.lo;
     if (aborted) v = __int_as_float(0x7fc00000);  // NaN: the step did not complete
     if (lane == 0 && (unsigned)step < (unsigned)a.jpart_rows) {
       const int nblk = gridDim.x * gridDim.y;
@@ -553,24 +554,24 @@ cudaError_t launch_project_batch(const SolveDev* solves, int count, int variant,
 // steps in turn took 8 us at the end of an N = 128 rollout).
 constexpr int kWarpBlocks = 1024;
 
-__device__ __forceinline__ void jreduce_body(const float* __restrict__ jpart, int nblk, int steps,
+__device__ __forceinline__ void jreduce_body(const double* __restrict__ jpart, int nblk, int steps,
                                              double* __restrict__ jsteps) {
   __shared__ double red[256];
   const int t = threadIdx.x;
   if (nblk <= kWarpBlocks) {
     const int s = blockIdx.x * 8 + t / 32;
     if (s >= steps) return;
-    const float* row = jpart + (size_t)s * nblk;
+    const double* row = jpart + (size_t)s * nblk;
     double v = 0.0;
-    for (int b = t % 32; b < nblk; b += 32) v += (double)gld(row + b);
+    for (int b = t % 32; b < nblk; b += 32) v += gld(row + b);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (t % 32 == 0) gst(jsteps + s, v);
     return;
   }
-  const float* row = jpart + (size_t)blockIdx.x * nblk;
+  const double* row = jpart + (size_t)blockIdx.x * nblk;
   double v = 0.0;
-  for (int b = t; b < nblk; b += 256) v += (double)gld(row + b);
+  for (int b = t; b < nblk; b += 256) v += gld(row + b);
   red[t] = v;
   __syncthreads();
   for (int h = 128; h > 0; h >>= 1) {
@@ -596,7 +597,7 @@ __device__ __forceinline__ void jfinal_body(const double* __restrict__ jsteps, i
   if (t == 0) gst(J, (float)red[0]);
 }
 
-__global__ void __launch_bounds__(256) k_jreduce(const float* __restrict__ jpart, int nblk, int steps,
+__global__ void __launch_bounds__(256) k_jreduce(const double* __restrict__ jpart, int nblk, int steps,
                                                  double* __restrict__ jsteps) {
   jreduce_body(jpart, nblk, steps, jsteps);
 }
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(256) k_jfinal(const double* __restrict__ jstep
   jfinal_body(jsteps, steps, jscale, J);
 }
 
-cudaError_t launch_jreduce(const float* jpart, int nblk, int steps, double* jsteps, float* J,
+cudaError_t launch_jreduce(const double* jpart, int nblk, int steps, double* jsteps, float* J,
                            double jscale, cudaStream_t st) {
   if (steps > 0) k_jreduce<<<jreduce_grid(nblk, steps), 256, 0, st>>>(jpart, nblk, steps, jsteps);
   k_jfinal<<<1, 256, 0, st>>>(jsteps, steps, jscale, J);

@@ -165,7 +165,7 @@ __device__ __forceinline__ void stencil_body(const StencilArgs& a, int step_off,
       v = warp_sum(v);
       if (tx == 0 && (unsigned)step < (unsigned)a.jpart_rows) {
         const int nblk = gx * gy;
-        gst(a.jpart + (size_t)step * nblk + by * gx + bx, v);
+        gst(a.jpart + (size_t)step * nblk + by * gx + bx, (double)v);
       }
     }
   }
@@ -377,9 +377,13 @@ __device__ __forceinline__ void stencil4_body(const StencilArgs& a, int step_off
     if (tid % 32 == 0) sRed[tid / 32] = jacc;
     __syncthreads();
     if (tid < 32) {
-      const float s = warp_sum(tid < NT / 32 ? sRed[tid] : 0.0f);
+      // a warp's 128 cells in float, 8 roundings deep as a 32 x 8 tile's 256; the
+      // warps' sums in double-float (error over the summed magnitudes at N = 512
+      // 1.5e-9 -> 5.7e-10, 9.4e-10 with tiles of 32 x 8)
+      DFloat s = {tid < NT / 32 ? sRed[tid] : 0.0f, 0.0f};
+      s = fold1(fold1(fold1(s, 4), 2), 1);
       if (tid == 0 && (unsigned)step < (unsigned)a.jpart_rows)
-        gst(a.jpart + (size_t)step * gx * gy + by * gx + bx, s);
+        gst(a.jpart + (size_t)step * gx * gy + by * gx + bx, (double)s.hi + (double)s.lo);
     }
   }
 }
