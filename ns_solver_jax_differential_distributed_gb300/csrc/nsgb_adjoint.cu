@@ -325,8 +325,10 @@ __device__ __forceinline__ void adjoint4_body(const AdjointArgs& a) {
     set4(sLy + 4 * e, ly);
   }
 
-  // theta sensitivities of the thread's own cells (adjoint_body): float over
-  // two cells, double-float across the block
+  // theta sensitivities of the thread's own cells (adjoint_body), summed in
+  // double-float from the first cell on: dJ/dnu is a small difference of large
+  // terms (the sums' rounding in float over two cells showed in it; the step
+  // took the same time)
   const int r = tid / (TW / 4), q = tid % (TW / 4) + 1;
   DFloat vA, vB, vN;
   {
@@ -340,21 +342,23 @@ __device__ __forceinline__ void adjoint4_body(const AdjointArgs& a) {
     get6(sUy + o, uy);
     get4(sUy + o - W4, vs);
     get4(sUy + o + W4, vn);
-    float fA[2] = {0.f, 0.f}, fB[2] = {0.f, 0.f}, fN[2] = {0.f, 0.f};
+    float fA[4], fB[4], fN[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int h = k / 2;
       const float ox = ux[k + 1], oy = uy[k + 1];
       const float w = fmaf(jscale, ox, dt * mx[k]);
-      fA[h] = fmaf(w, sDA[r], fA[h]);
-      fB[h] = fmaf(w, sDB[r], fB[h]);
+      fA[k] = w * sDA[r];
+      fB[k] = w * sDB[r];
       const float lux = ((us[k] - ox) + (un[k] - ox)) + ((ux[k + 2] - ox) + (ux[k] - ox));
       const float luy = ((vs[k] - oy) + (vn[k] - oy)) + ((uy[k + 2] - oy) + (uy[k] - oy));
-      fN[h] = fmaf(mx[k], lux, fmaf(my[k], luy, fN[h]));
+      fN[k] = fmaf(mx[k], lux, my[k] * luy);
     }
-    vA = df_add({fA[0], 0.f}, {fA[1], 0.f});
-    vB = df_add({fB[0], 0.f}, {fB[1], 0.f});
-    vN = df_add({fN[0], 0.f}, {fN[1], 0.f});
+    auto sum4 = [](const float (&f)[4]) {
+      return df_add(two_sum(f[0], f[1]), two_sum(f[2], f[3]));
+    };
+    vA = sum4(fA);
+    vB = sum4(fB);
+    vN = sum4(fN);
   }
   const int lane = tid & 31;
   // lanes 0-7: A, 16-23: B, 8-15 and 24-31: nu

@@ -314,6 +314,12 @@ __device__ __forceinline__ DFloat df_add(DFloat a, DFloat b) {
   return {hi, __fsub_rn(t, __fsub_rn(hi, s))};
 }
 
+// a + b of two floats, exactly (Knuth's TwoSum).
+__device__ __forceinline__ DFloat two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
+
 __device__ __forceinline__ DFloat warp_sum_df(DFloat v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
