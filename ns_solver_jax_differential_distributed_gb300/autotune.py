@@ -12,11 +12,12 @@ cold L2 for grids larger than L2) and keeps the fastest per stage:
 
 A plan that is not tuned starts from the library's measured defaults.  At the
 sizes of the resident kernel (N = 32 to 128), which runs at one shape only,
-the winner must also beat the default shape over a whole rollout.
+the winner must also beat the default shape over a whole rollout, and the
+adjoint's over a whole gradient.
 
-Results are cached in a JSON file keyed by GPU name, N and scheme
-(``$NSGB_TUNE_CACHE`` or ``<package>/_autotune/tiles.json``) so a process
-tunes a size once.  The stages are independent kernels, so each shape is
+Results are cached in a JSON file keyed by GPU name, N, scheme and the version
+of the shapes' meaning (``$NSGB_TUNE_CACHE`` or
+``<package>/_autotune/tiles.json``) so a process tunes a size once.  The stages are independent kernels, so each shape is
 tuned separately.
 """
 from __future__ import annotations
@@ -60,8 +61,13 @@ def _store(data: dict) -> None:
     os.replace(tmp, _CACHE_PATH)
 
 
+# Raised when kernels change so that shapes tuned before may no longer be the
+# fast ones (2: the resident kernel runs small grids at one shape).
+SHAPES_VERSION = 2
+
+
 def _key(N: int, scheme: str, device) -> str:
-    return f"{torch.cuda.get_device_name(device)}|N={N}|{scheme}"
+    return f"{torch.cuda.get_device_name(device)}|N={N}|{scheme}|v{SHAPES_VERSION}"
 
 
 # Row-streaming stencil: band widths (min(width, N) columns per CTA) and the
@@ -132,11 +138,11 @@ def _time_adjoint(u0, th, L, nu, dt, scheme, reps: int, steps: int = 6) -> float
 RESIDENT_MAX_N = 128  # largest grid of the resident kernel
 
 
-def _time_rollout(u0, th, L, nu, dt, scheme, steps: int = 64, reps: int = 3) -> float:
-    """Mean device ms per step of whole rollouts."""
-    def run():
-        return _native.op_rollout(u0, th, steps, L, nu, dt, _native.SCHEME_IDS[scheme], 0.5, 0.1, 1.0, True)
-    run()
+def _time_whole(run, u0, steps: int, reps: int = 3) -> float:
+    """Mean device ms per step of a whole solve (its second call captures the
+    graph later ones replay)."""
+    for _ in range(2):
+        run()
     torch.cuda.synchronize(u0.device)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
@@ -145,6 +151,15 @@ def _time_rollout(u0, th, L, nu, dt, scheme, steps: int = 64, reps: int = 3) -> 
     e1.record()
     torch.cuda.synchronize(u0.device)
     return e0.elapsed_time(e1) / (reps * steps)
+
+
+def _time_rollout(u0, th, L, nu, dt, scheme, steps: int = 64) -> float:
+    return _time_whole(lambda: _native.op_rollout(u0, th, steps, L, nu, dt, _native.SCHEME_IDS[scheme], 0.5, 0.1, 1.0,
+                                                  True), u0, steps)
+
+
+def _time_gradient(u0, th, L, nu, dt, scheme, steps: int = 64) -> float:
+    return _time_whole(lambda: _native.rollout_grad_raw(u0, th, steps, 1, L, nu, dt, scheme), u0, steps)
 
 
 def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, reps: int = 5,
@@ -168,6 +183,7 @@ def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, r
     cand = candidates(N, torch.cuda.get_device_properties(device).multi_processor_count)
     base = plan.tiles()
     base_radix = plan.fft_radix()
+    base_adj = plan.adjoint_tiles()  # (before a set_tiles, which also sets the adjoint's tile)
     results = {"stencil": {}, "rows": {}, "cols": {}}
     for (w, h) in cand["stencil"]:
         plan.set_tiles(w, h, base[2], base[3])
@@ -195,7 +211,6 @@ def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, r
     _apply(plan, best)
     # adjoint shapes: one backward step with the tuned FFT shapes
     results["adjoint"] = {}
-    base_adj = plan.adjoint_tiles()
     for (w, h) in cand["adjoint"]:
         plan.set_adjoint_tiles(w, h)
         results["adjoint"][(w, h)] = _time_adjoint(u0, th, L, nu, dt, scheme, max(2, reps // 2))
@@ -203,17 +218,28 @@ def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, r
     best["ms"]["adjoint_step"] = results["adjoint"][(best["adj_tw"], best["adj_th"])]
     best["default"] += list(base_adj)
     plan.set_adjoint_tiles(best["adj_tw"], best["adj_th"])
-    # Small grids: whole rollouts run as one resident launch at the plan's first
-    # shapes only, which no stage timing sees; keep those if they win as a whole.
+    # Small grids: whole solves run as one resident launch at a new plan's shapes
+    # only, which no stage timing sees; keep those where they win as a whole,
+    # the tile and the radix by rollouts, then the adjoint's tile by gradients.
     if N <= RESIDENT_MAX_N:
-        first = {"tw": base[0], "th": base[1], "rows": base[2], "cols": base[3], "radix_rows": base_radix[0],
-                 "radix_cols": base_radix[1], "adj_tw": base_adj[0], "adj_th": base_adj[1]}
-        tuned_ms = _time_rollout(u0, th, L, nu, dt, scheme)
-        _apply(plan, first)
-        first_ms = _time_rollout(u0, th, L, nu, dt, scheme)
-        if first_ms < tuned_ms:
+        new = _native.Plan(N, L, plan.device)
+        (tw, thh, rows, cols), (rr, rc) = new.tiles(), new.fft_radix()
+        adj = dict(zip(("adj_tw", "adj_th"), new.adjoint_tiles()))
+        first = {"tw": tw, "th": thh, "rows": rows, "cols": cols, "radix_rows": rr, "radix_cols": rc}
+        times = []
+        for shapes in (best, {**best, **first}):
+            _apply(plan, shapes)
+            times.append(_time_rollout(u0, th, L, nu, dt, scheme))
+        if times[1] < times[0]:
             best.update(first)
-        best["ms"]["rollout_step"] = min(first_ms, tuned_ms)
+        best["ms"]["rollout_step"] = min(times)
+        times = []
+        for shapes in (best, {**best, **adj}):
+            _apply(plan, shapes)
+            times.append(_time_gradient(u0, th, L, nu, dt, scheme))
+        if times[1] < times[0]:
+            best.update(adj)
+        best["ms"]["gradient_step"] = min(times)
         _apply(plan, best)
     if verbose:
         print(f"autotune N={N} {scheme}: best {best}")
