@@ -80,21 +80,29 @@ __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, flo
 }
 
 // ----------------------------------------------------------------- columns --
-// Spectral multiplier  -1/(k2x + k2y) * scale, 0 where the sum is 0.  The
-// hardware reciprocal (within one ulp) and one Newton-Raphson step,
-// r' = r + r (1 - d r) with a fused residual, give the correctly rounded 1/d
-// (the same float as __frcp_rn for every mantissa) without that function's
-// range check, which kept the 16 multipliers of a thread from overlapping;
-// host_wavenumbers keeps d in [1, 2^28].  FAST = false (N = 8192, whose 64
-// registers per thread the overlap would overflow) calls __frcp_rn.
+// 1/d for d in [1, 2^28] (host_wavenumbers): one Newton-Raphson step with a
+// fused residual, r' = r + r (1 - d r) (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990), from the PTX approximation r = (1 + e) / d, whose documented
+// error is at most 2^-23 on [1, 2), |e| <= 2^-22.  The residual is -e to 2^-24 of
+// itself, so r' is the rounding of (1 + x) / d with |x| <= 2^-44 + 2^-46: at most
+// (1/2 + 2^-19) ulp off.  For every mantissa and exponent of the range it is the
+// correctly rounded 1/d (tests/test_gpu_reciprocal.py).  The column pass of N =
+// 4096 with it and __frcp_rn in its place: 39.7 / 46.4 us.
+__device__ __forceinline__ float reciprocal(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return __fmaf_rn(r, __fmaf_rn(-d, r, 1.0f), r);
+}
+
+// Spectral multiplier  -1/(k2x + k2y) * scale, 0 where the sum is 0.  FAST =
+// false (N = 8192, whose 64 registers per thread the multipliers of a thread
+// overflow when they overlap) calls __frcp_rn.
 template <bool FAST>
 __device__ __forceinline__ float poisson_mult(float k2x, float k2y, float scale) {
   const float d = k2x + k2y;
   if constexpr (FAST) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = __fmaf_rn(r, __fmaf_rn(-d, r, 1.0f), r);
-    return d > 0.0f && d < INFINITY ? -r * scale : 0.0f;
+    return d > 0.0f && d < INFINITY ? -reciprocal(d) * scale : 0.0f;
   } else {
     const float inv = d == 0.0f ? 0.0f : __frcp_rn(d);
     return -inv * scale;
