@@ -120,6 +120,13 @@ int nsgb_plan_get_adjoint_tiles(const nsgb_plan* plan, int out[2]);
 int nsgb_plan_set_fused(nsgb_plan* plan, int rows);
 int nsgb_plan_get_fused(const nsgb_plan* plan, int* rows);
 
+/* No counterpart in the reference.  Whether the plan's rollouts (gradient = 0)
+ * or gradients (1) run as one resident launch on the stream (N = 32, 64, 128 at
+ * the launch shapes a plan starts with, on a stream that has the whole device):
+ * *clusters is the number of such solves the device runs at once, 0 where they
+ * run as separate launches. */
+int nsgb_plan_get_resident(const nsgb_plan* plan, int gradient, void* stream, int* clusters);
+
 /* Bytes of workspace for nsgb_poisson / nsgb_projector_step / nsgb_step. */
 size_t nsgb_poisson_workspace_bytes(const nsgb_plan* plan);
 size_t nsgb_step_workspace_bytes(const nsgb_plan* plan);

@@ -86,6 +86,7 @@ SIGNATURES = {
     "nsgb_plan_get_adjoint_tiles": ([_P, ctypes.POINTER(_I)], _I),
     "nsgb_plan_set_fused": ([_P, _I], _I),
     "nsgb_plan_get_fused": ([_P, ctypes.POINTER(_I)], _I),
+    "nsgb_plan_get_resident": ([_P, _I, _P, ctypes.POINTER(_I)], _I),
     "nsgb_poisson_workspace_bytes": ([_P], _S),
     "nsgb_step_workspace_bytes": ([_P], _S),
     "nsgb_rollout_workspace_bytes": ([_P, _I], _S),
@@ -212,6 +213,15 @@ class Plan:
         with torch.cuda.device(self.device):
             call("nsgb_plan_set_fused", self.handle, int(rows))
         self._ws.clear()
+
+    def resident_clusters(self, gradient: bool = False, stream: int | None = None) -> int:
+        """Solves that the device runs at once as resident launches on the
+        stream (default: the current one); 0: they run as separate launches."""
+        out = _I()
+        with torch.cuda.device(self.device):
+            call("nsgb_plan_get_resident", self.handle, int(bool(gradient)),
+                 stream_of(self.device) if stream is None else stream, ctypes.byref(out))
+        return int(out.value)
 
     def workspace(self, kind: str, nbytes: int, stream: int) -> torch.Tensor:
         """A cached uint8 workspace of at least nbytes for (kind, stream)."""

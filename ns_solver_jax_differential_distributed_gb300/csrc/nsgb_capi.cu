@@ -4,6 +4,8 @@
 // workspace of the size the *_workspace_bytes queries return.  A plan holds
 // the per-N constant tables and the launch shapes, and caches instantiated
 // CUDA graphs of rollout chunks.
+#include <cuda.h>
+
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -681,14 +683,34 @@ int plan_clusters(const nsgb_plan* plan) {
   return known[key] = resident_clusters(plan->N);
 }
 
-// Whether a plan's rollouts (grad: and gradients) run as resident launches: N
-// has an instance, the launch shapes are those it reproduces (32 x 8 tiles,
-// radix 16), and the device can place its clusters.
-bool resident_plan(const nsgb_plan* plan, bool grad) {
+// Whether a stream runs on its device's whole set of SMs, as far as the driver
+// can say: a stream of a green context has a share of them, which the count of
+// clusters above does not know and in which a cluster of 16 CTAs may have no
+// place.  (The query takes well under a microsecond.)
+bool whole_device(cudaStream_t st) {
+  using Query = CUresult (*)(CUstream, CUgreenCtx*);
+  static const Query query = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetGreenCtx", &fn, 12040, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      (void)cudaGetLastError();
+      fn = nullptr;
+    }
+    return (Query)fn;
+  }();
+  CUgreenCtx part = nullptr;
+  return !query || query((CUstream)st, &part) != CUDA_SUCCESS || !part;
+}
+
+// Whether a plan's rollouts (grad: and gradients) run as resident launches on a
+// stream: N has an instance, the launch shapes are those it reproduces (32 x 8
+// tiles, radix 16), and the device and the stream can place its clusters.
+bool resident_plan(const nsgb_plan* plan, bool grad, cudaStream_t st) {
   if (!resident_size(plan->N) || plan->radix_rows != 16 || plan->radix_cols != 16) return false;
   if (plan->tile_w != 32 || plan->tile_h != 8) return false;
   if (grad && (plan->adj_w != 32 || plan->adj_h != 8)) return false;
-  return plan_clusters(plan) > 0;
+  return whole_device(st) && plan_clusters(plan) > 0;
 }
 
 // Arguments of a rollout; gradient calls add theirs (resident_grad_args).
@@ -1104,6 +1126,13 @@ int nsgb_plan_get_fused(const nsgb_plan* plan, int* rows) {
   return NSGB_OK;
 }
 
+int nsgb_plan_get_resident(const nsgb_plan* plan, int gradient, void* stream, int* clusters) {
+  if (int r = check_plan(plan)) return r;
+  if (!clusters) return fail(NSGB_ERR_INVALID_ARG, "clusters is NULL");
+  *clusters = resident_plan(plan, gradient != 0, (cudaStream_t)stream) ? plan_clusters(plan) : 0;
+  return NSGB_OK;
+}
+
 int nsgb_plan_get_tiles(const nsgb_plan* plan, int out[4]) {
   if (int r = check_plan(plan)) return r;
   if (!out) return fail(NSGB_ERR_INVALID_ARG, "out is NULL");
@@ -1231,7 +1260,7 @@ int nsgb_step(const nsgb_plan* plan, const nsgb_phys* phys, const float* u, cons
   a.step_fixed = 0;
   a.t_from_step = 0;
   a.t_fixed = t;
-  if (resident_plan(plan, false)) {  // the five launches below in one
+  if (resident_plan(plan, false, st)) {  // the five launches below in one
     ResidentArgs r = resident_args(plan, a, w, 1);
     r.t_from_step = 0;
     r.t_fixed = t;
@@ -1280,7 +1309,7 @@ int nsgb_rollout(const nsgb_plan* plan_c, const nsgb_phys* phys, const float* u0
   }
 
   const double jscale = (double)phys->dt * (plan->L / plan->N) * (plan->L / plan->N);
-  if (resident_plan(plan, false)) {
+  if (resident_plan(plan, false, st)) {
     ResidentArgs r = resident_args(plan, a, w, steps);
     r.u0 = u0;
     r.u_final = u_final;
@@ -1574,7 +1603,7 @@ int nsgb_rollout_grad(const nsgb_plan* plan, const nsgb_phys* phys, const float*
   const int nblk = stencil_nblocks(plan->N, call.a.tw, call.a.th);
   const int adj_nblk = stencil_nblocks(plan->N, call.b.tw, call.b.th);
 
-  if (resident_plan(plan, true)) {
+  if (resident_plan(plan, true, st)) {
     call.a.theta = theta;
     ResidentArgs r = resident_grad_args(plan, call.a, g, steps, every, (phases & NSGB_GRAD_FORWARD) ? 0 : steps,
                                         (phases & NSGB_GRAD_BACKWARD) ? grad_ops_total(steps, every) : steps);
@@ -1828,7 +1857,7 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
     const nsgb_plan* plan = members[order[g0]].plan;
     int g1 = g0;
     while (g1 < count && members[order[g1]].plan == plan) ++g1;
-    if (resident_plan(plan, true) && g1 - g0 <= kResidentWaves * plan_clusters(plan)) {
+    if (resident_plan(plan, true, (cudaStream_t)stream) && g1 - g0 <= kResidentWaves * plan_clusters(plan)) {
       std::vector<ResidentArgs> tab[2];
       std::vector<GradAction> done;
       for (int q = g0; q < g1; ++q) {
