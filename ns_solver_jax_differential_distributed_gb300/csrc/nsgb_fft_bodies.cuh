@@ -88,7 +88,7 @@ __device__ __forceinline__ void rows_fwd_body(const float* __restrict__ rhs, flo
 // itself, so r' is the rounding of (1 + x) / d with |x| <= 2^-44 + 2^-46: at most
 // (1/2 + 2^-19) ulp off.  For every mantissa and exponent of the range it is the
 // correctly rounded 1/d (tests/test_gpu_reciprocal.py).  The column pass with it
-// and with __frcp_rn in its place: N = 4096 39.0 / 50.0 us, 1024 8.3 / 11.4.
+// and with __frcp_rn in its place: N = 4096 40.9 / 49.7 us, 1024 8.4 / 11.5.
 __device__ __forceinline__ float reciprocal(float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
@@ -135,15 +135,7 @@ __device__ __forceinline__ void cols_body(float2* __restrict__ spec, const float
   float g[E];
 #pragma unroll
   for (int s = 0; s < E; ++s) g[s] = poisson_mult<(N < 8192)>(gldg(k2 + j + s * T), k2y, scale);
-  if constexpr (N < 2048) {
-    fft::block_fft_scaled<N, true, E, BAR, R>(a, g, sb, j, tw);
-  } else {
-    // the products fuse into the first butterflies: 39.6 against 43.0 us at N =
-    // 4096
-#pragma unroll
-    for (int s = 0; s < E; ++s) a[s] = make_float2(a[s].x * g[s], a[s].y * g[s]);
-    fft::block_fft<N, true, E, BAR, R>(a, sb, j, tw);
-  }
+  fft::block_fft_scaled<N, true, E, BAR, R>(a, g, sb, j, tw);
   __syncthreads();  // rows clamped to N/2 were loaded by other threads
   if (kreq <= H) {
 #pragma unroll

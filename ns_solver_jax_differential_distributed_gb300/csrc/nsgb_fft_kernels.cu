@@ -28,10 +28,11 @@ namespace nsgb {
 // with two) and by shared memory; two CTAs of 256 threads per SM already
 // saturate both, so registers matter more than warps: the radix-16 kernel is
 // bounded to 80 registers (768 threads per SM), where the multipliers of a
-// thread overlap and little spills.  Times of the pass in the step: N = 4096
-// 46.4 -> 39.7 us, 1024 11.4 -> 8.2 us, 128 9.4 -> 6.3 us.  N = 8192 has CTAs of
-// 512 threads and needs two of them per SM (213 us, against 240 us for one with
-// 128 registers); so does radix 8, whose registers allow it.
+// thread overlap and little spills.  Times of the pass in the step, with 64
+// registers and a CUDA reciprocal before: N = 4096 46.4 -> 40.9 us, 1024 11.4 ->
+// 8.4 us.  N = 8192 has CTAs of 512 threads and needs two of them per SM (213 us,
+// against 240 us for one with 128 registers); so do threads of 8 values, whose
+// registers allow it.
 template <int N, int E>
 constexpr bool cols_two() {
   return E == 8 || N >= 8192;

@@ -26,6 +26,8 @@ CRC = {
     256: (0xcc83703f, 0x422887dc, 0xa04bbfe6),
     512: (0x128d9d60, 0x5f127dd0, 0x0b4fb3c9),
     1024: (0xbe5f468c, 0x5c5bb7b4, 0x489734d8),
+    2048: (0x5b943bfe, 0x3cf29b9c, 0xbc4518d3),
+    4096: (0x82283c54, 0xdb87ea30, 0x05e751bf),
 }
 
 
@@ -54,6 +56,11 @@ def results(nat, N):
 def test_default_results_keep_their_bits(nat, N):
     got = tuple(zlib.crc32(t.cpu().numpy().tobytes()) for t in results(nat, N))
     assert got == CRC[N], N
+
+
+def test_largest_poisson_solve_keeps_its_bits(nat):
+    rhs = _ints(8192, 1, -8, 9, 1.0)[0]
+    assert zlib.crc32(nat.op_poisson(rhs - rhs[0, 0], L).cpu().numpy().tobytes()) == 0x83e2d3d9
 
 
 @pytest.mark.parametrize("N,shape", [(128, (0, 64)), (256, (128, 32)), (256, (0, 32)), (256, (128, 0)), (512, (0, 16))])
