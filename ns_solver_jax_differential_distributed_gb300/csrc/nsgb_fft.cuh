@@ -103,23 +103,21 @@ __device__ __forceinline__ void dft(float2 (&a)[R]) {
   for (int k = 0; k < R; ++k) a[k] = b[k];
 }
 
-// Sum and difference of u g and v h: the first butterfly of a transform whose
-// inputs are multiplied by a spectral multiplier.  The products are rounded,
-// but for the second one of a transform's last pair (last), which is fused.
-// Spelled out, because the fusing a compiler finds for itself changes from
-// kernel to kernel and with it the last bits of a solve, and an upwind gradient
-// is not continuous in those: a cell of |u| below them takes the other
-// one-sided difference in the adjoint step.
-__device__ __forceinline__ void scaled_butterfly(float2 u, float g, float2 v, float h, bool last, float2& sum,
-                                                 float2& dif) {
-  const float ux = fmul(u.x, g), uy = fmul(u.y, g);
-  if (last) {
-    sum = make_float2(__fmaf_rn(v.x, h, ux), __fmaf_rn(v.y, h, uy));
-    dif = make_float2(__fmaf_rn(-v.x, h, ux), __fmaf_rn(-v.y, h, uy));
+// Sum and difference of u and v g, the last pair of the first stage of a
+// transform whose inputs are multiplied by a spectral multiplier: the products
+// of all other inputs are rounded, the last one's (fused) is not.  Spelled out,
+// because the fusing a compiler finds for itself changes from kernel to kernel
+// and with it the last bits of a solve, and an upwind gradient is not
+// continuous in those: a cell of |u| below them takes the other one-sided
+// difference in the adjoint step.
+__device__ __forceinline__ void scaled_butterfly(float2 u, float2 v, float g, bool fused, float2& sum, float2& dif) {
+  if (fused) {
+    sum = make_float2(__fmaf_rn(v.x, g, u.x), __fmaf_rn(v.y, g, u.y));
+    dif = make_float2(__fmaf_rn(-v.x, g, u.x), __fmaf_rn(-v.y, g, u.y));
   } else {
-    const float vx = fmul(v.x, h), vy = fmul(v.y, h);
-    sum = make_float2(fadd(ux, vx), fadd(uy, vy));
-    dif = make_float2(fsub(ux, vx), fsub(uy, vy));
+    const float x = fmul(v.x, g), y = fmul(v.y, g);
+    sum = make_float2(fadd(u.x, x), fadd(u.y, y));
+    dif = make_float2(fsub(u.x, x), fsub(u.y, y));
   }
 }
 
@@ -315,10 +313,10 @@ __device__ __forceinline__ void exchange_store(const float2 (&x)[CNT], float2* _
 // value is rounded as in a whole butterfly's registers, so the results are
 // those of radix 16 bit for bit, with twice the threads per transform and an
 // exchange through shared memory less than in radix 8.
-// SCALED: the inputs are multiplied by g (scaled_butterfly).  On return a[k] is
-// output 2 k + h.
+// SCALED: the last input still has its factor g to come (scaled_butterfly).  On
+// return a[k] is output 2 k + h.
 template <int N, int NS, bool INV, bool SCALED>
-__device__ __forceinline__ void half_butterfly(float2 (&a)[8], const float (&g)[8], int b, int h,
+__device__ __forceinline__ void half_butterfly(float2 (&a)[8], float g, int b, int h,
                                                const float2* __restrict__ tw) {
   constexpr int LX = N / 16 < 16 ? N / 16 : 16;  // the partner's lane, see split_index
   if constexpr (NS > 1) {
@@ -346,8 +344,8 @@ __device__ __forceinline__ void half_butterfly(float2 (&a)[8], const float (&g)[
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     float2 sum, dif;
-    if constexpr (SCALED) {
-      scaled_butterfly(a[s], g[s], a[s + 4], g[s + 4], h && s == 3, sum, dif);  // r = h + 2 s
+    if (SCALED && s == 3) {
+      scaled_butterfly(a[3], a[7], g, h, sum, dif);  // r = 15, or 14 if h = 0
     } else {
       sum = cadd(a[s], a[s + 4]);
       dif = csub(a[s], a[s + 4]);
@@ -382,9 +380,9 @@ __device__ __forceinline__ int split_index(int x) {
 
 // One Stockham pass (stride NS) and, recursively, the remaining passes: R the
 // radix, E values per thread, E = R or (radix 16) R / 2.  SCALED: the first
-// pass takes its inputs times g.
+// pass multiplies the last input by g.
 template <int N, int NS, bool INV, int E, int BAR, int R, bool SCALED>
-__device__ __forceinline__ void pass(float2 (&a)[E], const float (&g)[E], float2* __restrict__ sb, int j,
+__device__ __forceinline__ void pass(float2 (&a)[E], float g, float2* __restrict__ sb, int j,
                                      const float2* __restrict__ tw) {
   static_assert(E == R || (E == 8 && R == 16), "radix");
   constexpr int T = N / E;
@@ -405,10 +403,16 @@ __device__ __forceinline__ void pass(float2 (&a)[E], const float (&g)[E], float2
       for (int r = 0; r < RP; ++r) x[r] = a[q + r * Q];
       if constexpr (NS > 1) twiddle<NS, RP, R, INV>(x, b & (NS - 1), tw);
       if constexpr (SCALED) {
+        static_assert(Q == 1, "one butterfly per thread");
 #pragma unroll
         for (int t = 0; t < RP / 2; ++t) {
           float2 sum, dif;
-          scaled_butterfly(x[t], g[q + t * Q], x[t + RP / 2], g[q + (t + RP / 2) * Q], t == RP / 2 - 1, sum, dif);
+          if (t == RP / 2 - 1) {
+            scaled_butterfly(x[t], x[t + RP / 2], g, true, sum, dif);
+          } else {
+            sum = cadd(x[t], x[t + RP / 2]);
+            dif = csub(x[t], x[t + RP / 2]);
+          }
           x[t] = sum;
           x[t + RP / 2] = rot16<INV>(dif, t * (16 / RP));
         }
@@ -437,16 +441,18 @@ __device__ __forceinline__ void pass(float2 (&a)[E], const float (&g)[E], float2
 // (BAR = 0), or of the N/E-thread group synchronised by BAR, must call it (at
 // E < R every lane of the warp): it synchronises those threads between passes,
 // the last time after their last read of the exchange buffer, which is free
-// for reuse on return.  block_fft_scaled transforms a[s] * g[s].
+// for reuse on return.
 template <int N, bool INV, int E, int BAR = 0, int R = E>
 __device__ __forceinline__ void block_fft(float2 (&a)[E], float2* sb, int j, const float2* __restrict__ tw) {
-  const float none[E] = {};
-  pass<N, 1, INV, E, BAR, R, false>(a, none, sb, j, tw);
+  pass<N, 1, INV, E, BAR, R, false>(a, 0.0f, sb, j, tw);
 }
+// The transform of a[s] g[s].
 template <int N, bool INV, int E, int BAR = 0, int R = E>
 __device__ __forceinline__ void block_fft_scaled(float2 (&a)[E], const float (&g)[E], float2* sb, int j,
                                                  const float2* __restrict__ tw) {
-  pass<N, 1, INV, E, BAR, R, true>(a, g, sb, j, tw);
+#pragma unroll
+  for (int s = 0; s < E - 1; ++s) a[s] = make_float2(fmul(a[s].x, g[s]), fmul(a[s].y, g[s]));
+  pass<N, 1, INV, E, BAR, R, true>(a, g[E - 1], sb, j, tw);
 }
 
 }  // namespace fft
