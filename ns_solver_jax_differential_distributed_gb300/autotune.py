@@ -10,10 +10,11 @@ cold L2 for grids larger than L2) and keeps the fastest per stage:
   inverse),
 * Stockham radix and spectrum rows per CTA of the column FFT.
 
-A plan that is not tuned starts from the library's measured defaults.  At the
-sizes of the resident kernel (N = 32 to 128), which runs at one shape only,
-the winner must also beat the default shape over a whole rollout, and the
-adjoint's over a whole gradient.
+A plan that is not tuned starts from the library's measured defaults.  The
+winner must also beat those over a whole rollout, and the adjoint's shape over
+a whole gradient: a stage timed by itself does not share L2 with the others
+(N = 4096: bands of 512 x 72 won their stage, 176.5 us a step against 173.5 with
+the default), and the resident kernel (N = 32 to 128) runs at one shape only.
 
 Results are cached in a JSON file keyed by GPU name, N, scheme and the version
 of the shapes' meaning (``$NSGB_TUNE_CACHE`` or
@@ -135,9 +136,6 @@ def _time_adjoint(u0, th, L, nu, dt, scheme, reps: int, steps: int = 6) -> float
     return e0.elapsed_time(e1) / (reps * steps)
 
 
-RESIDENT_MAX_N = 128  # largest grid of the resident kernel
-
-
 def _time_whole(run, u0, steps: int, reps: int = 3) -> float:
     """Mean device ms per step of a whole solve (its second call captures the
     graph later ones replay)."""
@@ -153,12 +151,13 @@ def _time_whole(run, u0, steps: int, reps: int = 3) -> float:
     return e0.elapsed_time(e1) / (reps * steps)
 
 
-def _time_rollout(u0, th, L, nu, dt, scheme, steps: int = 64) -> float:
+def _time_rollout(u0, th, L, nu, dt, scheme, steps: int = 65) -> float:
     return _time_whole(lambda: _native.op_rollout(u0, th, steps, L, nu, dt, _native.SCHEME_IDS[scheme], 0.5, 0.1, 1.0,
                                                   True), u0, steps)
 
 
-def _time_gradient(u0, th, L, nu, dt, scheme, steps: int = 64) -> float:
+def _time_gradient(u0, th, L, nu, dt, scheme) -> float:
+    steps = 64 if u0.shape[-1] <= 512 else 8  # every state is kept
     return _time_whole(lambda: _native.rollout_grad_raw(u0, th, steps, 1, L, nu, dt, scheme), u0, steps)
 
 
@@ -218,29 +217,21 @@ def tune(N: int, L: float = 2 * math.pi, scheme: str = "central", device=None, r
     best["ms"]["adjoint_step"] = results["adjoint"][(best["adj_tw"], best["adj_th"])]
     best["default"] += list(base_adj)
     plan.set_adjoint_tiles(best["adj_tw"], best["adj_th"])
-    # Small grids: whole solves run as one resident launch at a new plan's shapes
-    # only, which no stage timing sees; keep those where they win as a whole,
-    # the tile and the radix by rollouts, then the adjoint's tile by gradients.
-    if N <= RESIDENT_MAX_N:
-        new = _native.Plan(N, L, plan.device)
-        (tw, thh, rows, cols), (rr, rc) = new.tiles(), new.fft_radix()
-        adj = dict(zip(("adj_tw", "adj_th"), new.adjoint_tiles()))
-        first = {"tw": tw, "th": thh, "rows": rows, "cols": cols, "radix_rows": rr, "radix_cols": rc}
+    # A new plan's shapes where whole solves are faster with them: the tile and
+    # the FFT shapes by rollouts, then the adjoint's tile by gradients.
+    new = _native.Plan(N, L, plan.device)
+    (tw, thh, rows, cols), (rr, rc) = new.tiles(), new.fft_radix()
+    first = {"tw": tw, "th": thh, "rows": rows, "cols": cols, "radix_rows": rr, "radix_cols": rc}
+    adj = dict(zip(("adj_tw", "adj_th"), new.adjoint_tiles()))
+    for shapes, timed, name in ((first, _time_rollout, "rollout_step"), (adj, _time_gradient, "gradient_step")):
         times = []
-        for shapes in (best, {**best, **first}):
-            _apply(plan, shapes)
-            times.append(_time_rollout(u0, th, L, nu, dt, scheme))
+        for cand in (best, {**best, **shapes}):
+            _apply(plan, cand)
+            times.append(timed(u0, th, L, nu, dt, scheme))
         if times[1] < times[0]:
-            best.update(first)
-        best["ms"]["rollout_step"] = min(times)
-        times = []
-        for shapes in (best, {**best, **adj}):
-            _apply(plan, shapes)
-            times.append(_time_gradient(u0, th, L, nu, dt, scheme))
-        if times[1] < times[0]:
-            best.update(adj)
-        best["ms"]["gradient_step"] = min(times)
-        _apply(plan, best)
+            best.update(shapes)
+        best["ms"][name] = min(times)
+    _apply(plan, best)
     if verbose:
         print(f"autotune N={N} {scheme}: best {best}")
         for kind, res in results.items():

@@ -1,6 +1,6 @@
-"""The autotuner at the resident kernel's sizes, with fake timings: it comes
-back to a new plan's shapes, the adjoint's among them, whenever whole solves
-are faster there, whatever the stage timings said, and it does not apply
+"""The autotuner with fake timings: it comes back to a new plan's shapes, the
+adjoint's among them, whenever whole solves are faster there, whatever the
+stage timings said (as at the resident kernel's sizes), and it does not apply
 shapes cached before the resident kernel."""
 import json
 
