@@ -84,17 +84,24 @@ __global__ void __launch_bounds__(1024) k_rows_inv_b(const SolveDev* __restrict_
 // Radix-16 passes by threads of 8 values (fft::half_butterfly) where a step
 // waits for the transforms' latency: the same bits from twice the threads.  Step
 // with whole / split butterflies, us: N = 16 8.7 / 7.5, 256 11.6 / 10.3 (rows
-// alone or columns alone 10.9; a batch of 8 15.7 / 14.1, of 30 29.2 / 30.4), 512,
-// columns only, 14.2 / 13.4 (batch of 11 39.7 / 41.1); from N = 1024 on it waits
-// for shared memory.  CTAs too large for twice the threads keep whole ones.
+// alone or columns alone 10.9), 512, columns only, 14.5 / 13.9; from N = 1024 on
+// it waits for shared memory.  So do batches of a million cells and more:
+// N = 256 x 8 15.6 / 14.2, x 16 20.4 / 20.2, x 20 23.0 / 23.1, x 30 29.3 / 30.0;
+// 512 x 3 19.7 / 19.3, x 4 21.4 / 21.5, x 6 26.9 / 27.5, x 11 39.7 / 41.0; but not
+// of smaller grids: 128 x 80 33.0 / 31.0, 64 x 300 35.2 / 32.2.  CTAs too large
+// for twice the threads keep whole butterflies.
 constexpr int kSplitRowsN = 256, kSplitColsN = 512;
 template <int N>
-static bool rows_split(const FftLaunch& L) {
-  return N <= kSplitRowsN && L.radix_rows == 16 && L.rows_per_cta / 2 * (N / 8) <= 1024;
+static bool split_pays(int count) {
+  return N < 256 || (size_t)count * N * N <= (size_t)1 << 20;
 }
 template <int N>
-static bool cols_split(const FftLaunch& L) {
-  return N <= kSplitColsN && L.radix_cols == 16 && L.cols_per_cta * (N / 8) <= 512;
+static bool rows_split(const FftLaunch& L, int count) {
+  return N <= kSplitRowsN && L.radix_rows == 16 && L.rows_per_cta / 2 * (N / 8) <= 1024 && split_pays<N>(count);
+}
+template <int N>
+static bool cols_split(const FftLaunch& L, int count) {
+  return N <= kSplitColsN && L.radix_cols == 16 && L.cols_per_cta * (N / 8) <= 512 && split_pays<N>(count);
 }
 
 template <int N, int R>
@@ -154,8 +161,8 @@ static cudaError_t stage_rows_inv(const FftLaunch& L, const SolveDev* sv, int co
 template <int N>
 static cudaError_t launch_poisson_fft(const FftLaunch& L, const SolveDev* sv, int count, cudaStream_t st) {
   constexpr int E = fft::ept(N);
-  const int r = rows_split<N>(L) ? 1 : L.radix_rows == 8 ? 2 : 0;
-  const int c = cols_split<N>(L) ? 1 : L.radix_cols == 8 ? 2 : 0;
+  const int r = rows_split<N>(L, count) ? 1 : L.radix_rows == 8 ? 2 : 0;
+  const int c = cols_split<N>(L, count) ? 1 : L.radix_cols == 8 ? 2 : 0;
   cudaError_t e = cudaSuccess;
   if (sv || L.rhs) {
     if constexpr (N <= kSplitRowsN)

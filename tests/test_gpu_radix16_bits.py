@@ -93,3 +93,18 @@ def test_persistent_ensemble_equals_default_plans(nat):
     torch.cuda.synchronize()
     for s, a, b in zip(specs, up, ur):
         assert torch.equal(a, b), (s.N, s.scheme)
+
+
+@pytest.mark.parametrize("N,count", [(256, 17), (512, 5)])
+def test_large_batches_give_the_same_bits(nat, N, count):
+    """Batches of more than a million cells run whole butterflies."""
+    from ns_solver_jax_differential_distributed_gb300 import ensemble
+    u0 = _ints(N, 2, -64, 65, 2.0 ** -6)
+    th = np.array([0.75, 0.5, 2.0 ** -10], np.float32)
+    for members in (1, count):
+        ens = ensemble.Ensemble([ensemble.SolveSpec(N, u0.cpu().numpy(), th, 2.0 ** -10, 2.0 ** -12, "upwind", L)] *
+                                members, steps=9, chunk=4)
+        us = [u.clone() for u in ens.run()[1]]
+        if members == 1:
+            want = us[0]
+        assert all(torch.equal(u, want) for u in us)
