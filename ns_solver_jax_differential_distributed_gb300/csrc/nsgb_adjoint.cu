@@ -22,8 +22,9 @@
 // adjoint kernel wrote rhs = div(lambda_{s+1}) / dt, the FFT kernels solved for
 // p, and this kernel applies mu = lambda - dt grad p on its tile.  The cell
 // arithmetic uses the folded coefficients of the fused forward step (dt/h,
-// dt nu/dx^2, 1/(h dt)) and FMAs; the theta sensitivities are summed in float
-// over a thread's few cells and in double from there on.
+// dt nu/dx^2, 1/(h dt)) and FMAs; the theta sensitivities are summed in
+// double-float, after float over a thread's few cells (one-cell tiles larger
+// than a block) or a row's four (bands), and in double across blocks and steps.
 #include "nsgb_adjoint_cell.cuh"
 #include "nsgb_rows.cuh"
 #include "nsgb_stencil_body.cuh"

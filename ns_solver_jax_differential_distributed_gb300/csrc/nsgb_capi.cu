@@ -1521,7 +1521,12 @@ struct GradCall {
 // Part 0 (forward_rest) or 1 (backward_rest) of a call, as a graph from the
 // second call with the same key on (an optimisation loop, a training loop over
 // changing inputs); one-off calls run eagerly, without the capture's host
-// cost.  Inside a caller's stream capture the launches are simply recorded.
+// cost.  The second call is a good time: capturing takes no longer than an eager
+// call in all but the shortest solves, and the third call has paid for it there
+// too.  First / second / later calls, ms: N = 256, 1000 steps, every 50 55.1 /
+// 45.8 / 28.8, 20 steps, every 7 1.15 / 1.31 / 0.65; N = 1024, 1000 steps, every 50
+// 95.5 / 82.5 / 67.7, 30 steps 2.05 / 1.94 / 1.50.  Inside a caller's stream
+// capture the launches are simply recorded.
 int grad_part(nsgb_plan* pl, const GradCall& call, int part, const void* ws, cudaStream_t st) {
   auto enqueue = [&](cudaStream_t s) { return part == 0 ? call.forward_rest(s) : call.backward_rest(s); };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1848,9 +1853,9 @@ int nsgb_grad_batch_advance(const nsgb_grad_member* members, int count, int ops,
   // Groups of small grids make all their operations in one resident launch
   // instead of four or five launches per tick (the same bits), as long as their
   // clusters run in kResidentWaves turns or fewer.  Measured, 180 operations of
-  // m members, ticks / resident: N = 32 m = 8 3.6 / 0.9 ms, m = 128 6.7 / 3.1;
-  // N = 64 m = 8 3.6 / 0.9, m = 64 5.5 / 4.3; N = 128 m = 4 3.5 / 1.1, m = 32
-  // 6.0 / 5.5, but m = 64 (about nine turns) 9.0 / 10.9.
+  // m members, ticks / resident: N = 32 m = 8 3.8 / 0.9 ms, m = 300 19.2 / 7.0;
+  // N = 64 m = 8 3.8 / 0.9, m = 60 6.2 / 3.8; N = 128 m = 4 3.6 / 1.0, m = 28
+  // 5.7 / 4.2, but m = 64 (about nine turns) 9.8 / 10.0.
   constexpr int kResidentWaves = 4;
   std::vector<char> resident(count, 0);
   for (int g0 = 0, gi = 0; g0 < count; ++gi) {
